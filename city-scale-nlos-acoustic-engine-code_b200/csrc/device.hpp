@@ -207,6 +207,47 @@ struct SchemeAArgs
                                //   storage row first read this many rows ahead
 };
 
+// Launch shape of the scheme-B FP32 step, two x-adjacent cells per thread:
+// blocks of four warps, each warp one 64-column segment of one row.  bx warps
+// lie along x (a template argument of the kernel) and 4 / bx along y; the
+// split that leaves the fewest warps without cells is taken, the widest one
+// where several do.  Four warps along x leave half of them idle in a row of
+// 128 columns: a 128^3 step took 80.5 us that way and 69.7 us with two, a
+// 97x83x41 step 25.7 and 22.8 us, a gradient step on 128^3 167 and 156 us.
+// The scheme-A and adjoint steps keep their blocks along x: they sit at their
+// register caps and the row index of a split block costs them 1-10 %.
+struct PairLaunch
+{
+    dim3 grid;
+    int bx;   // 4, 2 or 1
+};
+constexpr int kPairBlock = 128;
+inline PairLaunch pair_launch(const Layout& L)
+{
+    const long long seg = (L.nx + 63) / 64;
+    int best = 4;
+    long long least = 0;
+    for (int bx = 4; bx >= 1; bx /= 2)
+    {
+        const int by = 4 / bx;
+        const long long warps = ((seg + bx - 1) / bx * bx) * ((L.ny + by - 1) / by * by);
+        if (bx == 4 || warps < least) best = bx, least = warps;
+    }
+    const int by = 4 / best;
+    return PairLaunch{dim3((unsigned)((seg + best - 1) / best), (unsigned)((L.ny + by - 1) / by), (unsigned)L.nz), best};
+}
+#ifdef __CUDACC__
+// Column pair (0-based first column) and row (1-based) of a thread under pair_launch's shape with BX warps along x.
+template <int BX>
+__device__ __forceinline__ int pair_column() { return 2 * (int)(blockIdx.x * (32 * BX) + (threadIdx.x & (32 * BX - 1))); }
+template <int BX>
+__device__ __forceinline__ int pair_row()
+{
+    if (BX == 4) return blockIdx.y + 1;
+    return blockIdx.y * (4 / BX) + threadIdx.x / (32 * BX) + 1;
+}
+#endif
+
 // ---- launchers (kernels.cu) ----------------------------------------------
 // storage: 0 = float, 1 = __half.  All launches go to `stream`.
 cudaError_t launch_build_links(const uint8_t* mask_ref, uint32_t* links, uint32_t* near, const Layout& L,

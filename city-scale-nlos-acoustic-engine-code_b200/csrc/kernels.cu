@@ -245,8 +245,8 @@ __device__ __forceinline__ PairMoments pack_moments(float4 m0, float4 m1)
                         (v5 >> 4) | (v6 << 8) | (v7 << 20)}};
 }
 
-template <typename S, int BLOCK, int MINB, bool MOM = false>
-__global__ void __launch_bounds__(BLOCK, MINB) k_step(const S* __restrict__ fin, S* __restrict__ fout, Layout L,
+template <typename S, int BX, bool MOM = false>
+__global__ void __launch_bounds__(kPairBlock) k_step(const S* __restrict__ fin, S* __restrict__ fout, Layout L,
                                                       StepArgs a, float inv_scale,
                                                       PairMoments* __restrict__ mom = nullptr)
 {
@@ -254,11 +254,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_step(const S* __restrict__ fin,
     constexpr int BC = block_cells(sizeof(S));   // cells per interleaved block
     constexpr int BE = 19 * BC;                   // elements per block
     const int lane = threadIdx.x & 31;
-    const int c0r = 2 * (blockIdx.x * BLOCK + threadIdx.x);   // first column (0-based) of the pair
+    const int c0r = pair_column<BX>();                        // first column (0-based) of the pair
     const bool active = c0r < L.nx;
     const int c0 = active ? c0r : ((L.nx - 1) & ~1);         // inactive lanes shadow a valid pair
-    const int j = blockIdx.y + 1;
+    const int j = pair_row<BX>();
     const int k = blockIdx.z + 1;
+    if (BX < 4 && j > L.ny) return;   // whole warps
     const long long e0 = L.elem(0, c0 + 1, j, k);
     const S* own = fin + e0;
     const long long rs = L.row_stride, ps = L.plane_stride;
@@ -1274,10 +1275,6 @@ static_assert(sizeof(g_field_scratch) == sizeof(float) * LBM_NOALLOC_MAX_CELLS,
               "the static field array must hold the grid size lbm_get_rho_noalloc accepts");
 
 dim3 row_grid(const Layout& L) { return dim3((unsigned)((L.nx + 127) / 128), (unsigned)L.ny, (unsigned)L.nz); }
-dim3 pair_grid(const Layout& L, int block)
-{
-    return dim3((unsigned)(((L.nx + 1) / 2 + block - 1) / block), (unsigned)L.ny, (unsigned)L.nz);
-}
 
 // Warp-pipelined FP16 step: dynamic shared memory (one ring per warp) and a
 // grid of as many CTAs as the GPU holds at once (every warp then walks rows
@@ -1323,13 +1320,14 @@ cudaError_t launch_hw(const __half* fin, __half* fout, const Layout& L, const St
     return cudaGetLastError();
 }
 
-template <typename S>
-cudaError_t launch_step_t(const S* fin, S* fout, const Layout& L, const StepArgs& a, float inv_scale,
-                          cudaStream_t stream)
+template <bool MOM>
+cudaError_t launch_pair_step(const float* fin, float* fout, const Layout& L, const StepArgs& a, PairMoments* mom,
+                             cudaStream_t stream)
 {
-    if constexpr (std::is_same<S, __half>::value)
-        return launch_hw<2, 4, 5>(fin, fout, L, a, inv_scale, stream);
-    k_step<S, 128, 0><<<pair_grid(L, 128), 128, 0, stream>>>(fin, fout, L, a, inv_scale);
+    const PairLaunch g = pair_launch(L);
+    if (g.bx == 4) k_step<float, 4, MOM><<<g.grid, kPairBlock, 0, stream>>>(fin, fout, L, a, 1.0f, mom);
+    else if (g.bx == 2) k_step<float, 2, MOM><<<g.grid, kPairBlock, 0, stream>>>(fin, fout, L, a, 1.0f, mom);
+    else k_step<float, 1, MOM><<<g.grid, kPairBlock, 0, stream>>>(fin, fout, L, a, 1.0f, mom);
     return cudaGetLastError();
 }
 
@@ -1394,15 +1392,14 @@ cudaError_t prepare_step(int storage)
 cudaError_t launch_step(int storage, const void* fin, void* fout, const Layout& L, const StepArgs& a,
                         float scale, cudaStream_t stream)
 {
-    if (storage == 0) return launch_step_t<float>((const float*)fin, (float*)fout, L, a, 1.0f, stream);
-    return launch_step_t<__half>((const __half*)fin, (__half*)fout, L, a, 1.0f / scale, stream);
+    if (storage == 0) return launch_pair_step<false>((const float*)fin, (float*)fout, L, a, nullptr, stream);
+    return launch_hw<2, 4, 5>((const __half*)fin, (__half*)fout, L, a, 1.0f / scale, stream);
 }
 
 cudaError_t launch_step_moments(const float* fin, float* fout, const Layout& L, const StepArgs& a,
                                 PairMoments* mom, cudaStream_t stream)
 {
-    k_step<float, 128, 0, true><<<pair_grid(L, 128), 128, 0, stream>>>(fin, fout, L, a, 1.0f, mom);
-    return cudaGetLastError();
+    return launch_pair_step<true>(fin, fout, L, a, mom, stream);
 }
 
 cudaError_t launch_source(int storage, void* f, const Layout& L, const StepArgs& sa, const SourceArgs& a,

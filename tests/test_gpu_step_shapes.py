@@ -1,0 +1,62 @@
+"""The fused step's launch shapes against the FP64 oracle at the sizes where a
+row's columns or a plane's rows do not fill a block: one warp and less per row,
+two, three, four and five 64-column segments, odd widths, and row counts that
+leave rows of a block without cells.
+
+Tolerances: those of tests/test_gpu_parity.py for FP32 and FP16 storage.
+"""
+import numpy as np
+import pytest
+
+import nlos_lbm
+import oracle
+import scenarios
+from nlos_lbm import abi
+from scenarios import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+FP32_PROBE_TOL = 1e-5
+FP32_STATE_TOL = 1e-4
+FP16_PROBE_TOL = 1e-3
+
+SIZES = [(17, 9, 7), (33, 10, 8), (63, 11, 9), (64, 8, 12), (65, 13, 6), (97, 9, 10), (128, 10, 9), (129, 6, 11),
+         (191, 7, 8), (257, 5, 7), (320, 6, 6)]
+
+
+def case(size, storage, ground):
+    """A box crossing a segment edge, a source against the low x face, open faces (and a ground plane)."""
+    nx, ny, nz = size
+    faces = [abi.LBM_BC_NSCBC] * 6
+    if ground:
+        faces[abi.FACE_ZLO] = abi.LBM_BC_WALL
+    cfg = scenarios.lattice_config(nx, ny, nz, 0.52, face_bc=tuple(faces), sponge_faces=(1 << 6) - 1,
+                                   sponge_width=2.0, storage=storage, f16_scale=1e5)
+    x0 = min(60, nx // 2)
+    tris = scenarios.boxes_to_triangles([(x0, ny // 2, 0, min(x0 + 6, nx - 1), ny - 1, nz // 2)])
+    src = abi.reference_source(sx=2.3, sy=2.1, sz=nz / 2 + 0.2, ex=2.3, ey=2.1, ez=nz / 2 + 0.2, amp=1e-3,
+                               freq=1 / 20.0, waveform=abi.LBM_WAVE_SINE)
+    far = abi.reference_source(sx=nx - 1.6, sy=ny / 2, sz=nz - 2.2, ex=nx / 2, ey=1.4, ez=nz - 1.2, speed=0.3, amp=1e-3,
+                               freq=1 / 16.0, waveform=abi.LBM_WAVE_SINE, injection=abi.LBM_INJECT_TRILINEAR)
+    probes = np.array([[0.5, 2.5, nz / 2], [3.5, 3.5, nz / 2], [nx - 0.5, ny / 2, nz - 1.5],
+                       [nx - 2.5, 1.5, nz - 0.5], [1.5, 0.5, nz - 0.5]])
+    return cfg, [src, far], probes, tris
+
+
+@pytest.mark.parametrize("size", SIZES, ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("storage", [abi.LBM_STORE_F32, abi.LBM_STORE_F16], ids=["f32", "f16"])
+def test_step_matches_oracle(size, storage, gpu):
+    steps = 24
+    cfg, srcs, probes, tris = case(size, storage, ground=size[2] % 2 == 0)
+    g = nlos_lbm.Solver(cfg, srcs, probes, triangles=tris)
+    o = oracle.OracleSolver(cfg, srcs, probes, triangles=tris)
+    assert np.array_equal(g.get_mask(), o.get_mask())
+    g.step(steps)
+    o.step(steps)
+    assert rel_l2(g.get_probes(), o.get_probes()) <= (FP32_PROBE_TOL if storage == abi.LBM_STORE_F32 else FP16_PROBE_TOL)
+    if storage == abi.LBM_STORE_F32:
+        w = np.array(abi.W)
+        nx, ny, nz = g.dims_halo
+        dg, do = (s.get_f().reshape(nz, ny, nx, 19)[1:-1, 1:-1, 1:-1] - w for s in (g, o))
+        assert np.max(np.abs(dg - do)) <= FP32_STATE_TOL * np.max(np.abs(do))
+    g.close()
