@@ -94,7 +94,12 @@ struct lbm_handle
     uint32_t* links = nullptr;
     uint32_t* near = nullptr;
     float* sig = nullptr;              // sig_x | sig_y | sig_z
-    XFace xf{nullptr, nullptr};        // x-face exports and ghosts
+    XFace xf{nullptr, nullptr};        // x-face exports and (both parities') ghosts
+    // x-face ghosts of each population buffer: a batched step reads its own buffer's and writes the next
+    // one's.  A z-slab steps by single calls only and keeps one array, which its messages write into.
+    float* xgh_par[2] = {nullptr, nullptr};
+    int xgh_last = 0;                  // which of them was filled last (lbm_get_f)
+    SourceNext* d_next = nullptr;      // [2] sources applied by the batched step that reads buffer 0 / 1
     StepArgs sa{};
     GhostArgs ga{};
     Control* ctl = nullptr;            // device
@@ -122,7 +127,6 @@ struct lbm_handle
     // scheme A (family 01-04): omega and source-weight profiles, x-face arrays of both parities
     SchemeAArgs aa{};
     float* a_prof = nullptr;           // om_x | om_y | om_z | fld_x | fld_y | fld_z
-    float* xgh_par[2] = {nullptr, nullptr};
     bool scheme_a() const { return cfg.scheme == LBM_SCHEME_A; }
 
     // z-slab exchange between handles of one process: message buffers
@@ -182,6 +186,7 @@ struct lbm_handle
         cudaFree(a_prof); a_prof = nullptr;
         cudaFree(ctl); ctl = nullptr;
         cudaFree(d_table); d_table = nullptr;
+        cudaFree(d_next); d_next = nullptr;
         cudaFree(d_probe_ijk); d_probe_ijk = nullptr;
         cudaFree(d_probe_out); d_probe_out = nullptr;
         cudaFree(d_energy); d_energy = nullptr;
@@ -209,6 +214,14 @@ struct lbm_handle
     }
 
     int nprobe() const { return (int)probe_xyz.size() / 3; }
+    // x-face arrays and step arguments of population buffer `parity`
+    XFace xface(int parity) const { return XFace{xf.xexp, xgh_par[parity]}; }
+    StepArgs step_args(int parity) const
+    {
+        StepArgs a = sa;
+        a.xf = xface(parity);
+        return a;
+    }
 };
 
 // ---------------------------------------------------------------- helpers
@@ -953,9 +966,10 @@ extern "C" int lbm_init(lbm_handle* h)
     h->sig = dalloc<float>((size_t)nxs + ny + nz, e);
     const size_t n_xexp = (size_t)2 * Q * ny * nz, n_xgh = (size_t)2 * Q * nyt * nzt;
     h->xf.xexp = dalloc<float>(n_xexp, e);
-    const size_t n_xgh_all = n_xgh * (h->scheme_a() ? 2 : 1);   // scheme A: one array per step parity
+    const size_t n_xgh_all = n_xgh * (h->slab ? 1 : 2);   // one array per population buffer
     h->xf.xgh = dalloc<float>(n_xgh_all, e);
     h->ctl = dalloc<Control>(1, e);
+    h->d_next = dalloc<SourceNext>(2, e);
     if (e != cudaSuccess) return h->cuda_fail(e, "device allocation");
     CK(cudaMemsetAsync(h->ctl, 0, sizeof(Control), h->stream), "memset control");
     CK(cudaMemsetAsync(h->links, 0, cells * sizeof(uint32_t), h->stream), "memset links");
@@ -963,7 +977,8 @@ extern "C" int lbm_init(lbm_handle* h)
     CK(cudaMemsetAsync(h->xf.xexp, 0, n_xexp * sizeof(float), h->stream), "memset x faces");
     CK(cudaMemsetAsync(h->xf.xgh, 0, n_xgh_all * sizeof(float), h->stream), "memset x faces");
     h->xgh_par[0] = h->xf.xgh;
-    h->xgh_par[1] = h->xf.xgh + (h->scheme_a() ? n_xgh : 0);
+    h->xgh_par[1] = h->xf.xgh + (h->slab ? 0 : n_xgh);
+    h->xgh_last = 0;
     CK(cudaMallocHost(&h->ctl_host, sizeof(Control)), "cudaMallocHost");
     *h->ctl_host = Control{};
     CK(cudaMemsetAsync(h->sig, 0, (size_t)nxs * 4, h->stream), "memset sponge");
@@ -1100,6 +1115,7 @@ extern "C" int lbm_init(lbm_handle* h)
 
 namespace {
 
+// (a batched launch reads the schedule row of the device step counter)
 SourceArgs source_args(lbm_handle* h, bool batched)
 {
     SourceArgs a{};
@@ -1122,7 +1138,7 @@ SourceArgs source_args(lbm_handle* h, bool batched)
     return a;
 }
 
-ProbeArgs probe_args(lbm_handle* h, bool batched, long long direct_row)
+ProbeArgs probe_args(lbm_handle* h, bool batched, long long direct_row, int parity = 0)
 {
     ProbeArgs a{};
     a.n = h->nprobe();
@@ -1130,6 +1146,7 @@ ProbeArgs probe_args(lbm_handle* h, bool batched, long long direct_row)
     a.out = h->d_probe_out;
     a.energy = h->d_energy;
     a.ctl = batched ? h->ctl : nullptr;
+    a.parity = parity;
     a.direct_row = direct_row;
     a.scale = h->scale;
     a.nonfinite = &h->ctl->nonfinite;
@@ -1146,6 +1163,7 @@ void scheme_a_args(lbm_handle* h, int parity, bool batched, long long s, StepArg
     b = h->aa;
     b.table = h->d_table;
     b.ctl = batched ? h->ctl : nullptr;
+    b.parity = parity;
     b.xgh_out = h->xgh_par[parity ^ 1];
     b.mass_direct[0] = b.mass_direct[1] = 0.f;
     if (!batched && b.field_mode >= 0)
@@ -1156,13 +1174,54 @@ void scheme_a_args(lbm_handle* h, int parity, bool batched, long long s, StepArg
     }
 }
 
-// The fused step of the handle's scheme from buffer `parity` into the other,
+// Whether a batched scheme-B step is one launch (the next step's sources and
+// ghosts applied to its results) or three (source, ghost fill, step).  One
+// launch saves the small kernels and the gaps between them, 7 us a step and
+// more, but its step kernel is 4-6 % slower (registers, and the x faces' ghosts
+// are one lane's work), so the line lies where the two are equal: measured
+// fused / separate, FP32 64^3 10.7 / 16.9 us, 128^3 66.9 / 72.8,
+// 200x160x100 101 / 109, 256x256x128 219 / 224, 333x222x111 247 / 232,
+// 512x512x128 904 / 891; FP16 64^3 11.5 / 21.5, 128^3 51 / 66, 256x256x128
+// 154 / 167, 400x300x128 281 / 282, 512x512x128 562 / 555.
+bool fused_steps(const lbm_handle* h)
+{
+    const long long most = h->storage == LBM_STORE_F16 ? 1LL << 23 : 1LL << 22;
+    return (long long)h->L.nx * h->L.ny * h->L.nz <= most;
+}
+
+// Faces whose ghosts follow the characteristic boundary, as FusedArgs::open.
+unsigned open_faces(const lbm_handle* h)
+{
+    unsigned m = 0;
+    for (int f = 0; f < h->ga.nfaces; ++f) m |= 1u << (h->ga.face[f].axis * 2 + h->ga.face[f].side);
+    return m;
+}
+
+// Arguments of the batched scheme-B step that reads buffer `parity`.
+FusedArgs fused_args(lbm_handle* h, int parity)
+{
+    FusedArgs fa{};
+    fa.open = open_faces(h);
+    fa.xgh_out = h->xgh_par[parity ^ 1];
+    fa.next = h->d_next + parity;
+    fa.prep = h->d_next + (parity ^ 1);
+    fa.ctl = h->ctl;
+    fa.parity = parity;
+    fa.src = source_args(h, true);
+    fa.probe = probe_args(h, true, 0, parity);
+    return fa;
+}
+
+// The step of the handle's scheme from buffer `parity` into the other,
 // bracketed by timing events when kernel timing is on.
 cudaError_t timed_step_launch(lbm_handle* h, int parity, bool batched, long long s)
 {
     const auto launch = [&]() {
+        if (!h->scheme_a() && batched)
+            return launch_batched_step(h->storage, h->f[parity], h->f[parity ^ 1], h->L, h->step_args(parity), h->scale,
+                                       fused_args(h, parity), fused_steps(h), h->stream);
         if (!h->scheme_a())
-            return launch_step(h->storage, h->f[parity], h->f[parity ^ 1], h->L, h->sa, h->scale,
+            return launch_step(h->storage, h->f[parity], h->f[parity ^ 1], h->L, h->step_args(parity), h->scale,
                                h->stream);
         StepArgs sa;
         SchemeAArgs b;
@@ -1211,13 +1270,31 @@ int harvest_timing(lbm_handle* h)
     return LBM_OK;
 }
 
-// One full time step on the device (source -> ghosts -> fused step ->
-// probes), reading the step index from the device control block.
-cudaError_t enqueue_batched_step(lbm_handle* h, int parity, int& kernels, bool captured = false)
+// Before the first step of a batch (scheme B): its source and ghost fill, and
+// the sources its step applies; every later step's are applied by the step
+// before it.
+cudaError_t enqueue_batch_start(lbm_handle* h, int& kernels)
+{
+    const int p = h->cur;
+    kernels = 1;
+    cudaError_t e = launch_source(h->storage, h->f[p], h->L, h->step_args(p), source_args(h, true), p, h->d_next + p,
+                                  h->stream);
+    if (e == cudaSuccess && h->ga.total > 0)
+    {
+        GhostArgs g = h->ga;
+        g.xf = h->xface(p);
+        e = launch_ghost(h->storage, h->f[p], h->L, g, h->stream);
+        kernels++;
+    }
+    return e;
+}
+
+// One full time step on the device, reading the step index from the device
+// control block.
+cudaError_t enqueue_batched_step(lbm_handle* h, int parity, int& kernels)
 {
     cudaError_t e = cudaSuccess;
     void* fc = h->f[parity];
-    void* fn = h->f[parity ^ 1];
     kernels = 0;
     if (h->scheme_a())
     {
@@ -1230,50 +1307,33 @@ cudaError_t enqueue_batched_step(lbm_handle* h, int parity, int& kernels, bool c
         kernels++;
         if (b.copy)
         {
-            e = launch_copy_a((const float*)fc, (float*)fn, h->L, sa, b, h->stream);
+            e = launch_copy_a((const float*)fc, (float*)h->f[parity ^ 1], h->L, sa, b, h->stream);
             if (e != cudaSuccess) return e;
             kernels++;
         }
-        e = launch_probe_a((const float*)fc, h->L, sa, b, probe_args(h, true, 0), h->stream);
+        e = launch_probe_a((const float*)fc, h->L, sa, b, probe_args(h, true, 0, parity), h->stream);
         kernels++;
         return e;
     }
-    if (!h->srcs.empty())
+    if (!fused_steps(h))
     {
-        e = launch_source(h->storage, fc, h->L, h->sa, source_args(h, true), h->stream);
-        if (e != cudaSuccess) return e;
-        kernels++;
+        const StepArgs sa = h->step_args(parity);
+        if (!h->srcs.empty())
+        {
+            e = launch_source(h->storage, fc, h->L, sa, source_args(h, true), parity, nullptr, h->stream);
+            kernels++;
+        }
+        if (e == cudaSuccess && h->ga.total > 0)
+        {
+            GhostArgs g = h->ga;
+            g.xf = sa.xf;
+            e = launch_ghost(h->storage, fc, h->L, g, h->stream);
+            kernels++;
+        }
     }
-    if (h->ga.total > 0)
-    {
-        e = launch_ghost(h->storage, fc, h->L, h->ga, h->stream);
-        if (e != cudaSuccess) return e;
-        kernels++;
-    }
-    if (!captured)
-    {
-        e = timed_step_launch(h, parity, true, 0);
-        if (e != cudaSuccess) return e;
-        kernels++;
-        e = launch_probe(h->storage, fc, h->L, h->sa, probe_args(h, true, 0), h->stream);
-        kernels++;
-        return e;
-    }
-    // In the captured graph the probe record, which reads this step's input
-    // buffer and ghosts (the step only reads them) and advances the device step
-    // counter (no scheme-B step kernel reads it), is a branch beside the step,
-    // joined before the next step's source reads the counter.  Direct launches
-    // of single steps keep one stream (no graph amortises the fork and join).
-    e = cudaEventRecord(h->ev_fork, h->stream);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->ev_fork, 0);
-    if (e == cudaSuccess) e = launch_probe(h->storage, fc, h->L, h->sa, probe_args(h, true, 0), h->side);
-    if (e == cudaSuccess) e = cudaEventRecord(h->ev_join, h->side);
-    if (e != cudaSuccess) return e;
+    if (e == cudaSuccess) e = timed_step_launch(h, parity, true, 0);
     kernels++;
-    e = timed_step_launch(h, parity, true, 0);
-    if (e != cudaSuccess) return e;
-    kernels++;
-    return cudaStreamWaitEvent(h->stream, h->ev_join, 0);
+    return e;
 }
 
 int build_graph(lbm_handle* h)
@@ -1283,8 +1343,8 @@ int build_graph(lbm_handle* h)
     cudaError_t e = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return h->cuda_fail(e, "begin capture");
     int k0 = 0, k1 = 0;
-    cudaError_t le = enqueue_batched_step(h, 0, k0, true);
-    if (le == cudaSuccess) le = enqueue_batched_step(h, 1, k1, true);
+    cudaError_t le = enqueue_batched_step(h, 0, k0);
+    if (le == cudaSuccess) le = enqueue_batched_step(h, 1, k1);
     e = cudaStreamEndCapture(h->stream, &g);
     if (le != cudaSuccess) e = le;
     if (e == cudaSuccess) e = cudaGraphInstantiate(&h->graph, g, 0);
@@ -1436,7 +1496,8 @@ void field_rho_initial(const lbm_handle* h, float* out, size_t n)
 // (float)(rho - 1) of the last step into d (device, interior cells).
 cudaError_t field_rho_last_step(lbm_handle* h, float* d)
 {
-    if (!h->scheme_a()) return launch_field_rho(h->storage, h->f[h->cur ^ 1], d, h->L, h->sa, h->scale, h->stream);
+    if (!h->scheme_a())
+        return launch_field_rho(h->storage, h->f[h->cur ^ 1], d, h->L, h->step_args(h->cur ^ 1), h->scale, h->stream);
     StepArgs sa;
     SchemeAArgs b;
     scheme_a_args(h, h->cur ^ 1, false, h->step - 1, sa, b);
@@ -1454,7 +1515,7 @@ int reset_halos_if_dirty(lbm_handle* h)
     const size_t nloc = (size_t)(L.nx + 2) * (L.ny + 2) * (L.nz + 2);
     double* d = nullptr;
     CK(cudaMalloc(&d, nloc * Q * sizeof(double)), "halo reset");
-    cudaError_t e = launch_export_f(h->storage, h->f[h->cur], d, L, h->xf, h->scale, h->stream);
+    cudaError_t e = launch_export_f(h->storage, h->f[h->cur], d, L, h->xface(h->xgh_last), h->scale, h->stream);
     if (e == cudaSuccess)
     {
         tmp.resize(nloc * Q);
@@ -1473,7 +1534,7 @@ int reset_halos_if_dirty(lbm_handle* h)
                     for (int q = 0; q < Q; ++q) tmp[idx * Q + q] = wd(q);
                 }
         e = cudaMemcpyAsync(d, tmp.data(), nloc * Q * sizeof(double), cudaMemcpyHostToDevice, h->stream);
-        if (e == cudaSuccess) e = launch_import_f(h->storage, h->f[h->cur], d, L, h->xf, h->scale, h->stream);
+        if (e == cudaSuccess) e = launch_import_f(h->storage, h->f[h->cur], d, L, h->xface(h->cur), h->scale, h->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     }
     cudaFree(d);
@@ -1496,7 +1557,7 @@ extern "C" int lbm_apply_source(lbm_handle* h, double t)
     CK(cudaSetDevice(h->device), "cudaSetDevice");
     SourceArgs a = source_args(h, false);
     for (size_t s = 0; s < h->srcs.size(); ++s) a.direct[s] = entry_for(h, h->srcs[s], t);
-    CK(launch_source(h->storage, h->f[h->cur], h->L, h->sa, a, h->stream), "source kernel");
+    CK(launch_source(h->storage, h->f[h->cur], h->L, h->step_args(h->cur), a, 0, nullptr, h->stream), "source kernel");
     h->launches++;
     return LBM_OK;
 }
@@ -1511,7 +1572,10 @@ extern "C" int lbm_exchange_halos(lbm_handle* h)
     if (st) return st;
     if (h->ga.total > 0)
     {
-        CK(launch_ghost(h->storage, h->f[h->cur], h->L, h->ga, h->stream), "ghost kernel");
+        GhostArgs g = h->ga;
+        g.xf = h->xface(h->cur);
+        CK(launch_ghost(h->storage, h->f[h->cur], h->L, g, h->stream), "ghost kernel");
+        h->xgh_last = h->cur;
         h->launches++;
     }
     return LBM_OK;
@@ -1532,6 +1596,7 @@ extern "C" int lbm_step_collision_bgk(lbm_handle* h)
         CK(launch_copy_a((const float*)h->f[h->cur], (float*)h->f[h->cur ^ 1], h->L, sa, b, h->stream), "halo copy");
         h->launches++;
     }
+    h->xgh_last = h->cur;
     h->cur ^= 1;
     h->step++;
     return harvest_timing(h);
@@ -1561,8 +1626,8 @@ extern "C" int lbm_record_probes(lbm_handle* h)
     }
     else
     {
-        CK(launch_probe(h->storage, h->f[h->cur ^ 1], h->L, h->sa, probe_args(h, false, h->probe_pending),
-                        h->stream),
+        CK(launch_probe(h->storage, h->f[h->cur ^ 1], h->L, h->step_args(h->cur ^ 1),
+                        probe_args(h, false, h->probe_pending), h->stream),
            "probe kernel");
     }
     h->launches++;
@@ -1580,6 +1645,25 @@ extern "C" int lbm_step(lbm_handle* h, int nsteps)
     st = reset_halos_if_dirty(h);
     if (st) return st;
     const int np = h->nprobe();
+    if (h->slab)
+    {
+        // a z-slab takes its halo planes from messages between single calls; steps without them run the
+        // same calls one by one
+        for (int n = 0; n < nsteps; ++n)
+        {
+            st = lbm_apply_source(h, (double)h->step * h->dt);
+            if (!st) st = lbm_exchange_halos(h);
+            if (!st) st = lbm_step_collision_bgk(h);
+            if (!st) st = lbm_record_probes(h);
+            if (st) return st;
+        }
+        CK(cudaMemcpyAsync(&h->ctl_host->nonfinite, &h->ctl->nonfinite, sizeof(int), cudaMemcpyDeviceToHost, h->stream),
+           "probe flag");
+        CK(cudaStreamSynchronize(h->stream), "step sync");
+        if (h->ctl_host->nonfinite)
+            return h->fail(LBM_ERR_NAN, "non-finite probe value by step " + std::to_string(h->step));
+        return LBM_OK;
+    }
     const bool use_graph = h->cfg.use_graphs && !h->timing;
     long long left = nsteps;
     while (left > 0)
@@ -1598,7 +1682,8 @@ extern "C" int lbm_step(lbm_handle* h, int nsteps)
             if (st) return st;
             continue;
         }
-        h->ctl_host->step = h->step;
+        h->ctl_host->step[0] = h->ctl_host->step[1] = h->step;
+        h->ctl_host->last = h->step + chunk - 1;
         h->ctl_host->table_base = h->table_base;
         // the probe row of step s is s - probe_base: rows continue after the
         // ones already buffered
@@ -1607,6 +1692,12 @@ extern "C" int lbm_step(lbm_handle* h, int nsteps)
            "control");
         h->h2d_bytes += (long)offsetof(Control, nonfinite);
         long long done = 0;
+        if (!h->scheme_a() && fused_steps(h))
+        {
+            int k = 0;
+            CK(enqueue_batch_start(h, k), "batch start");
+            h->launches += k;
+        }
         while (done < chunk)
         {
             if (use_graph && h->cur == 0 && chunk - done >= 2)
@@ -1634,6 +1725,7 @@ extern "C" int lbm_step(lbm_handle* h, int nsteps)
                "probe flag");
             h->d2h_bytes += (long)sizeof(int);
         }
+        h->xgh_last = h->cur ^ 1;
         // the control block upload must not be overwritten before the copy ran
         CK(cudaStreamSynchronize(h->stream), "step sync");
         h->step += chunk;
@@ -1799,7 +1891,7 @@ extern "C" int lbm_get_f(lbm_handle* h, double* out, long capacity)
     CK(cudaSetDevice(h->device), "cudaSetDevice");
     double* d = nullptr;
     CK(cudaMalloc(&d, n * sizeof(double)), "f export buffer");
-    cudaError_t e = launch_export_f(h->storage, h->f[h->cur], d, L, h->xf, h->scale, h->stream);
+    cudaError_t e = launch_export_f(h->storage, h->f[h->cur], d, L, h->xface(h->xgh_last), h->scale, h->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, d, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
     h->d2h_bytes += (long)(n * sizeof(double));
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
@@ -1822,10 +1914,11 @@ extern "C" int lbm_set_f(lbm_handle* h, const double* in, long count)
     CK(cudaMalloc(&d, n * sizeof(double)), "f import buffer");
     cudaError_t e = cudaMemcpyAsync(d, in, n * sizeof(double), cudaMemcpyHostToDevice, h->stream);
     h->h2d_bytes += (long)(n * sizeof(double));
-    if (e == cudaSuccess) e = launch_import_f(h->storage, h->f[h->cur], d, L, h->xf, h->scale, h->stream);
+    if (e == cudaSuccess) e = launch_import_f(h->storage, h->f[h->cur], d, L, h->xface(h->cur), h->scale, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     cudaFree(d);
     if (e != cudaSuccess) return h->cuda_fail(e, "set_f");
+    h->xgh_last = h->cur;
     h->launches++;
     h->halo_dirty = true;
     return LBM_OK;
@@ -2029,7 +2122,7 @@ int rest_state(lbm_handle* h)
     const size_t n_xexp = (size_t)2 * Q * h->L.ny * h->L.nz, n_xgh = (size_t)2 * Q * (h->L.ny + 2) * (h->L.nz + 2);
     for (int b = 0; b < 2; ++b) CK(cudaMemsetAsync(h->f[b], 0, pop_bytes, h->stream), "rest state");
     CK(cudaMemsetAsync(h->xf.xexp, 0, n_xexp * sizeof(float), h->stream), "rest state");
-    CK(cudaMemsetAsync(h->xf.xgh, 0, n_xgh * sizeof(float), h->stream), "rest state");
+    CK(cudaMemsetAsync(h->xf.xgh, 0, 2 * n_xgh * sizeof(float), h->stream), "rest state");
     CK(cudaMemsetAsync(h->d_energy, 0, (size_t)std::max(h->nprobe(), 1) * sizeof(double), h->stream), "rest state");
     CK(cudaStreamSynchronize(h->stream), "rest state");
     h->step = 0;
@@ -2397,17 +2490,19 @@ extern "C" int lbm_adjoint_grad(lbm_handle* h, int nsteps, const double* observe
         {
             r = cudaEventRecord(h->ev_fork, h->stream);
             if (r == cudaSuccess) r = cudaStreamWaitEvent(h->side, h->ev_fork, 0);
-            if (r == cudaSuccess) r = launch_source(h->storage, h->f[h->cur], L, h->sa, sargs, h->side);
+            if (r == cudaSuccess) r = launch_source(h->storage, h->f[h->cur], L, h->step_args(h->cur), sargs, 0, nullptr, h->side);
             if (r == cudaSuccess) r = cudaEventRecord(h->ev_join, h->side);
         }
         else
         {
-            r = launch_source(h->storage, h->f[h->cur], L, h->sa, sargs, h->stream);
+            r = launch_source(h->storage, h->f[h->cur], L, h->step_args(h->cur), sargs, 0, nullptr, h->stream);
         }
         kernels++;
         if (r == cudaSuccess && h->ga.total > 0)
         {
-            r = launch_ghost(h->storage, h->f[h->cur], L, g, h->stream);
+            GhostArgs gp = g;
+            gp.xf = h->xface(h->cur);
+            r = launch_ghost(h->storage, h->f[h->cur], L, gp, h->stream);
             kernels++;
         }
         if (r == cudaSuccess && beside) r = cudaStreamWaitEvent(h->stream, h->ev_join, 0);
@@ -2423,7 +2518,7 @@ extern "C" int lbm_adjoint_grad(lbm_handle* h, int nsteps, const double* observe
         pa.out = d_pred;
         cudaError_t r = cudaEventRecord(h->ev_fork, h->stream);
         if (r == cudaSuccess) r = cudaStreamWaitEvent(h->side, h->ev_fork, 0);
-        if (r == cudaSuccess) r = launch_probe(h->storage, h->f[h->cur], L, h->sa, pa, h->side);
+        if (r == cudaSuccess) r = launch_probe(h->storage, h->f[h->cur], L, h->step_args(h->cur), pa, h->side);
         if (r == cudaSuccess) r = cudaEventRecord(h->ev_join, h->side);
         kernels++;
         return r;
@@ -2431,7 +2526,7 @@ extern "C" int lbm_adjoint_grad(lbm_handle* h, int nsteps, const double* observe
     const auto collide = [&](int s, bool probe) {
         cudaError_t r = probe ? probe_beside(s) : cudaSuccess;
         if (r == cudaSuccess)
-            r = launch_step(h->storage, h->f[h->cur], h->f[h->cur ^ 1], L, h->sa, h->scale, h->stream);
+            r = launch_step(h->storage, h->f[h->cur], h->f[h->cur ^ 1], L, h->step_args(h->cur), h->scale, h->stream);
         kernels++;
         if (r == cudaSuccess && probe) r = cudaStreamWaitEvent(h->stream, h->ev_join, 0);
         h->cur ^= 1;
@@ -2450,7 +2545,7 @@ extern "C" int lbm_adjoint_grad(lbm_handle* h, int nsteps, const double* observe
         kernels++;
         cudaError_t r = probe_step >= 0 ? probe_beside(probe_step) : cudaSuccess;
         if (r == cudaSuccess)
-            r = launch_step_moments((const float*)h->f[h->cur], (float*)h->f[h->cur ^ 1], L, h->sa, mom_of(slot),
+            r = launch_step_moments((const float*)h->f[h->cur], (float*)h->f[h->cur ^ 1], L, h->step_args(h->cur), mom_of(slot),
                                     h->stream);
         if (r == cudaSuccess && probe_step >= 0) r = cudaStreamWaitEvent(h->stream, h->ev_join, 0);
         h->cur ^= 1;
@@ -2631,7 +2726,7 @@ cudaError_t slab_msg(lbm_handle* h, bool pack, int side, void* msg)
     const Layout& L = h->L;
     const int k = pack ? (side ? L.nz : 1) : (side ? L.nz + 1 : 0);
     const int up = pack ? side : 1 - side;
-    return launch_slab_msg(pack, h->f[h->cur], h->xf.xgh, msg, L, k, up, h->storage == LBM_STORE_F16 ? 2 : 4,
+    return launch_slab_msg(pack, h->f[h->cur], h->xgh_par[h->cur], msg, L, k, up, h->storage == LBM_STORE_F16 ? 2 : 4,
                            h->stream);
 }
 

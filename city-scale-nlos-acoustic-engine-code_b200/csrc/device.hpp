@@ -66,7 +66,11 @@ struct Layout
 // Device control block: read by the kernels of a batched (graph) step.
 struct Control
 {
-    long long step;        // time step index of the step being executed
+    // time step index of the step being executed: a step that reads population
+    // buffer p reads step[p] and sets step[p ^ 1] for the next one, so no block
+    // reads the word that another block of the same launch writes
+    long long step[2];
+    long long last;        // last step of this batch of steps
     long long table_base;  // step index of source-table row 0
     long long probe_base;  // step index of probe-buffer row 0
     int nonfinite;         // set by the probe kernels when an owned probe reads a non-finite value
@@ -98,6 +102,21 @@ struct SourceArgs
     double x_min, y_min, z_min, dx;   // origin of the whole grid
     float scale;
     int k_off;                         // first z-layer of this handle's slab (0: the whole grid)
+};
+
+// Sources of one step as amounts per cell, computed a step ahead (epilogue.cuh): what the step
+// before it adds to its results.
+constexpr int kStencilCells = 343;     // (2 R + 1)^3 at the largest radius 3
+struct SourceBox
+{
+    int i0, j0, k0, n;                 // first cell (halo-inclusive) and extent; n = 0: nothing injected
+};
+struct SourceNext
+{
+    int fill;                          // 0: the step leaves its results as they are (last step of a batch)
+    int pad[3];
+    SourceBox box[kMaxSources];
+    float4 add[kMaxSources][kStencilCells];   // per cell, i fastest: gains of directions 0, 1-6, 7-18; w = 1: FLUID
 };
 
 struct GhostFace
@@ -155,10 +174,31 @@ struct ProbeArgs
     const int* ijk;            // [n][3] halo-inclusive cell coordinates; i = -1: not owned
     double* out;               // [row][n], row = step - probe_base
     double* energy;            // [n] running sum of p^2 (FP64)
-    Control* ctl;              // nullptr: row = direct_row, no counter update
+    Control* ctl;              // nullptr: row = direct_row, else ctl->step[parity] - ctl->probe_base
+    int parity;
     long long direct_row;
     float scale;
     int* nonfinite;            // set to 1 when an owned probe reads a non-finite value
+};
+
+// What a batched scheme-B step does beside and after its own update
+// (epilogue.cuh): its first blocks record the probes of the step and advance
+// the step counter.  A fused step's also prepare the sources of the step after
+// the next, and every warp adds the next step's sources to its results and, at
+// the open faces, writes the next step's ghosts.
+struct FusedArgs
+{
+    unsigned open;             // bit f: face f is a characteristic (NSCBC) face
+    float* xgh_out;            // x-face ghosts of the next step
+    const SourceNext* next;    // sources of the next step
+    SourceNext* prep;          // receives those of the step after it
+    Control* ctl;              // step counter and last step; nullptr: direct_step, direct_last
+    int parity;                // population buffer the step reads
+    long long direct_step, direct_last;
+    SourceArgs src;
+    ProbeArgs probe;           // n = 0: no probe record in this step
+    float4* face_mom;          // non-null: moments of the next step's ghosts' interior cells, as GhostArgs::face_mom
+    long long face_first[6];   // first ghost of face f in that order
 };
 
 // Scheme A (the reference's 01-04 family).  The stored state is the
@@ -192,6 +232,7 @@ struct SchemeAArgs
     float u0sq;                // u0 . u0
     const SourceEntry* table;  // schedule rows [row][nsrc] (row = step - ctl->table_base), as SourceArgs
     const Control* ctl;        // nullptr: use mass_direct
+    int parity;                // step counter ctl->step[parity]
     float mass_direct[2];      // mass of step s and of step s + 1 (direct launches)
     float* xgh_out;            // x-halo values written for the next step
     int copy;                  // zero-gradient halos on every face
@@ -252,13 +293,19 @@ __device__ __forceinline__ int pair_row()
 // storage: 0 = float, 1 = __half.  All launches go to `stream`.
 cudaError_t launch_build_links(const uint8_t* mask_ref, uint32_t* links, uint32_t* near, const Layout& L,
                                cudaStream_t stream);
+// Source injection of one step; next non-null (first step of a batch of fused steps): also prepares the
+// sources of the step after it.
 cudaError_t launch_source(int storage, void* f, const Layout& L, const StepArgs& sa, const SourceArgs& a,
-                          cudaStream_t stream);
+                          int parity, SourceNext* next, cudaStream_t stream);
 cudaError_t launch_ghost(int storage, void* f, const Layout& L, const GhostArgs& a, cudaStream_t stream);
 // Fused step: FP32 storage runs the two-cells-per-thread pair kernel, FP16
 // storage the warp pipelines of cp.async copies.
 cudaError_t launch_step(int storage, const void* fin, void* fout, const Layout& L, const StepArgs& a,
                         float scale, cudaStream_t stream);
+// A batched step: the same with the probes recorded and the step counter advanced; fused: also with the next
+// step's sources and ghosts applied to its results.
+cudaError_t launch_batched_step(int storage, const void* fin, void* fout, const Layout& L, const StepArgs& a,
+                                float scale, const FusedArgs& fa, bool fused, cudaStream_t stream);
 // One-time set-up of the fused step on the current device (shared-memory
 // attribute, occupancy); call before the first launch or capture.
 cudaError_t prepare_step(int storage);

@@ -13,6 +13,7 @@
 
 #include "check.cuh"
 #include "device.hpp"
+#include "epilogue.cuh"
 #include "lattice.cuh"
 
 namespace lbm {
@@ -95,23 +96,6 @@ struct PairIo<__half>
     static __device__ __forceinline__ float2 right(V cur, unsigned next) { return cvt(__byte_perm(cur, next, 0x5432)); }
     static __device__ __forceinline__ float rnd(float v) { return __half2float(__float2half_rn(v)); }
 };
-
-__device__ __forceinline__ void moments(const float (&G)[Q], float& rho, float& jx, float& jy, float& jz)
-{
-    rho = 0.f;
-    jx = jy = jz = 0.f;
-#pragma unroll
-    for (int q = 0; q < Q; ++q)
-    {
-        rho += G[q];
-        if (ex(q) > 0) jx += G[q];
-        if (ex(q) < 0) jx -= G[q];
-        if (ey(q) > 0) jy += G[q];
-        if (ey(q) < 0) jy -= G[q];
-        if (ez(q) > 0) jz += G[q];
-        if (ez(q) < 0) jz -= G[q];
-    }
-}
 
 __device__ __forceinline__ uint32_t near_bits(const StepArgs& a, const Layout& L, int col, int j, int k)
 {
@@ -217,6 +201,109 @@ __device__ __forceinline__ void collide2(float2 (&G)[Q], float inv_scale, float 
     }
 }
 
+// What a step launch does beyond the update: nothing (single calls); the
+// blocks beside it (probe record, step counter); those and the next step's
+// sources and ghosts.
+enum StepMode { kPlain = 0, kSide = 1, kFused = 2 };
+
+// Blocks beside a batched step's own: block 0 prepares the sources of the step
+// after the next (fused) and advances the step counter, the others record this
+// step's probes, a warp each.  They read what the step only reads.
+__host__ __device__ constexpr int side_blocks(int nprobe, int warps) { return 1 + (nprobe + warps - 1) / warps; }
+
+template <typename S, int MODE>
+__device__ __forceinline__ void side_block(const S* __restrict__ fin, const Layout& L, const StepArgs& a,
+                                           const FusedArgs& fa, int block, double* red)
+{
+    const long long s = fa.ctl ? fa.ctl->step[fa.parity] : fa.direct_step;
+    [[maybe_unused]] const long long last = fa.ctl ? fa.ctl->last : fa.direct_last;
+    if (block == 0)
+    {
+        if (MODE == kFused) prepare_sources(fa.prep, fa.src, s + 2, s + 1 < last, L, a.links, red);
+        if (fa.ctl && threadIdx.x == 0) fa.ctl->step[fa.parity ^ 1] = s + 1;
+        return;
+    }
+    const int p = (block - 1) * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5);
+    if (p < fa.probe.n)
+        probe_warp<S>(fin, L, a.links, a.xf.xgh, fa.probe, fa.ctl ? s - fa.ctl->probe_base : fa.probe.direct_row, p,
+                      threadIdx.x & 31);
+}
+
+// The next step's sources on a pair's results (kernel of FP32 storage).
+__device__ __forceinline__ void add_sources(float2 (&G)[Q], const SourceNext* __restrict__ nx, unsigned sources, int c0,
+                                            int j, int k, const Layout& L)
+{
+    while (sources)
+    {
+        const int s = __ffs(sources) - 1;
+        sources &= sources - 1;
+        const SourceBox b = nx->box[s];
+        const int row = ((k - b.k0) * b.n + (j - b.j0)) * b.n, d = c0 + 1 - b.i0;
+        const bool in0 = d >= 0 && d < b.n, in1 = d + 1 >= 0 && d + 1 < b.n && c0 + 1 < L.nx;
+        float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
+        if (in0) a0 = nx->add[s][row + d];
+        if (in1) a1 = nx->add[s][row + d + 1];
+        if (a0.w != 0.f)
+        {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) G[q].x += source_gain(a0, q);
+        }
+        if (a1.w != 0.f)
+        {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) G[q].y += source_gain(a1, q);
+        }
+    }
+}
+
+// The next step's ghosts of an open y or z face from a pair's results; `ghost`
+// is the pair's place in the halo row.
+template <int AXIS, int SIDE>
+__device__ __forceinline__ void ghost_pair(const float2 (&G)[Q], const float4& m0, const float4& m1, float* ghost)
+{
+    constexpr int BC = block_cells(sizeof(float));
+    float2 o[Q];
+    nscbc<AXIS, SIDE>(m0, 1.0f, [&](int q) { return G[q].x; }, [&](int q, float v) { o[q].x = v; });
+    nscbc<AXIS, SIDE>(m1, 1.0f, [&](int q) { return G[q].y; }, [&](int q, float v) { o[q].y = v; });
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+        if (inward<AXIS, SIDE>(q)) *reinterpret_cast<float2*>(ghost + q * BC) = o[q];
+}
+// ... and of an open x face, from the cell at the row's end.
+template <int SIDE, typename Get>
+__device__ __forceinline__ void ghost_end(const float4& m, float inv_scale, const FusedArgs& fa, const XFace& xf,
+                                          const Layout& L, int j, int k, Get&& get)
+{
+    nscbc<0, SIDE>(m, inv_scale, get, [&](int q, float v) { fa.xgh_out[xf.gh_index(SIDE, q, j, k, L.ny, L.nz)] = v; });
+}
+
+// Moments of the ghosts' interior cells, for the adjoint: the pair (c0, c0 + 1)
+// of row (j, k), `row` its open y and z faces, `ends` the x faces that its first
+// (bits 0-1) and second cell (bits 2-3) border.
+__device__ __forceinline__ void keep_face_moments(const FusedArgs& fa, const Layout& L, unsigned row, unsigned ends, int c0,
+                                                  int j, int k, const float4& m0, const float4& m1)
+{
+    const long long xc = (long long)(k - 1) * L.ny + (j - 1), yc = (long long)(k - 1) * L.nx + c0,
+                    zc = (long long)(j - 1) * L.nx + c0;
+#pragma unroll
+    for (int f = 2; f < 6; ++f)
+    {
+        if (!((row >> f) & 1u)) continue;
+        float4* p = fa.face_mom + fa.face_first[f] + (f < 4 ? yc : zc);
+        p[0] = m0;
+        if (c0 + 1 < L.nx) p[1] = m1;
+    }
+    if (ends & 1u) fa.face_mom[fa.face_first[0] + xc] = m0;
+    if (ends & 2u) fa.face_mom[fa.face_first[1] + xc] = m0;
+    if (ends & 8u) fa.face_mom[fa.face_first[1] + xc] = m1;
+}
+
+// Open y and z faces that row (j, k) borders.
+__device__ __forceinline__ unsigned row_faces(unsigned open, int j, int k, const Layout& L)
+{
+    return open & ((j == 1 ? 4u : 0u) | (j == L.ny ? 8u : 0u) | (k == 1 ? 16u : 0u) | (k == L.nz ? 32u : 0u));
+}
+
 // Fused pull-stream + halfway bounce-back + BGK + sponge (06:906-972), two
 // x-adjacent cells per thread.  Direction q of the pair comes from the row
 // (j - ey, k - ez) of the block-interleaved layout as one aligned vector at
@@ -245,12 +332,28 @@ __device__ __forceinline__ PairMoments pack_moments(float4 m0, float4 m1)
                         (v5 >> 4) | (v6 << 8) | (v7 << 20)}};
 }
 
-template <typename S, int BX, bool MOM = false>
-__global__ void __launch_bounds__(kPairBlock) k_step(const S* __restrict__ fin, S* __restrict__ fout, Layout L,
-                                                      StepArgs a, float inv_scale,
-                                                      PairMoments* __restrict__ mom = nullptr)
+// MODE: the first zx layers of blocks are the blocks beside the step; a fused
+// step writes the x-face exports only where its results stay as they are.
+// 80 registers (24 warps per SM) for the fused step: at the plain step's 72 it
+// spills 40 bytes, 256x256x128 233 us a step against 218; at 96 250 us.
+template <int BX, bool MOM, int MODE>
+__global__ void __launch_bounds__(kPairBlock, MODE == kFused ? 6 : 0) k_step(const float* __restrict__ fin, float* __restrict__ fout, Layout L,
+                                                      StepArgs a, PairMoments* __restrict__ mom,
+                                                      const __grid_constant__ FusedArgs fa, int zx)
 {
+    using S = float;
     using P = PairIo<S>;
+    constexpr bool FUSED = MODE == kFused;
+    if constexpr (MODE != kPlain)
+    {
+        if ((int)blockIdx.z < zx)
+        {
+            __shared__ double red[16];
+            const int block = (int)((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
+            if (block < side_blocks(fa.probe.n, kPairBlock / 32)) side_block<S, MODE>(fin, L, a, fa, block, red);
+            return;
+        }
+    }
     constexpr int BC = block_cells(sizeof(S));   // cells per interleaved block
     constexpr int BE = 19 * BC;                   // elements per block
     const int lane = threadIdx.x & 31;
@@ -258,7 +361,7 @@ __global__ void __launch_bounds__(kPairBlock) k_step(const S* __restrict__ fin, 
     const bool active = c0r < L.nx;
     const int c0 = active ? c0r : ((L.nx - 1) & ~1);         // inactive lanes shadow a valid pair
     const int j = pair_row<BX>();
-    const int k = blockIdx.z + 1;
+    const int k = (int)blockIdx.z - (MODE != kPlain ? zx : 0) + 1;
     if (BX < 4 && j > L.ny) return;   // whole warps
     const long long e0 = L.elem(0, c0 + 1, j, k);
     const S* own = fin + e0;
@@ -279,7 +382,6 @@ __global__ void __launch_bounds__(kPairBlock) k_step(const S* __restrict__ fin, 
         if (b & 2u) lk1 = a.links[cl + 1];
     }
     const bool any_link = __any_sync(kFull, (lk0 | lk1) != 0u);
-
     float2 G[Q];
 #pragma unroll
     for (int q = 0; q < Q; ++q)
@@ -320,6 +422,17 @@ __global__ void __launch_bounds__(kPairBlock) k_step(const S* __restrict__ fin, 
             }
         }
     }
+    // FUSED: bits 0-7 the sources whose cells the row holds, bit 8 that results take sources and ghosts at all
+    unsigned todo = 0u;
+    if constexpr (FUSED)
+    {
+        if (fa.next->fill != 0)
+        {
+            todo = 256u;
+            if (fa.src.nsrc > 0) todo |= sources_of_row(fa.next, fa.src.nsrc, lane, j, k);
+        }
+    }
+
     // x faces: sources in the x halo come from the x-face ghosts.
     const bool xlo = active && c0 == 0;
     const bool xhi0 = active && c0 == L.nx - 1;       // nx odd: first cell of the pair is the last
@@ -340,7 +453,7 @@ __global__ void __launch_bounds__(kPairBlock) k_step(const S* __restrict__ fin, 
 
     const float syz = fmaxf(a.sig_y[j - 1], a.sig_z[k - 1]);
     const float2 sg = make_float2(fmaxf(a.sig_x[c0], syz), fmaxf(c0 + 1 < L.nx ? a.sig_x[c0 + 1] : 0.f, syz));
-    collide2(G, inv_scale, a.omega, sg, (lk0 & kSolidSelfBit) != 0u, (lk1 & kSolidSelfBit) != 0u,
+    collide2(G, 1.0f, a.omega, sg, (lk0 & kSolidSelfBit) != 0u, (lk1 & kSolidSelfBit) != 0u,
              [&](float2 rho, float2 jx, float2 jy, float2 jz) {
                  if constexpr (MOM)
                  {
@@ -352,9 +465,34 @@ __global__ void __launch_bounds__(kPairBlock) k_step(const S* __restrict__ fin, 
              });
 
     S* out = fout + e0;
+    if (FUSED && (todo & 255u)) add_sources(G, fa.next, todo & 255u, c0, j, k, L);
 #pragma unroll
     for (int q = 0; q < Q; ++q)
         if (LBM_IN(kChkStepStore, e0 + q * BC, L.total - 1)) P::st(out + q * BC, G[q]);
+
+    if constexpr (FUSED)
+    {
+        if (todo & 256u)
+        {
+            const unsigned row = row_faces(fa.open, j, k, L);
+            const unsigned ends = (xlo ? fa.open & 1u : 0u) | (xhi0 ? fa.open & 2u : 0u) | (xhi1 ? (fa.open & 2u) << 2 : 0u);
+            if (!(row | ends)) return;
+            // a row's end takes the moments of its own cell only, unless the whole row is a face
+            float4 m0 = make_float4(0.f, 0.f, 0.f, 0.f), m1 = m0;
+            if (row | (ends & 3u)) m0 = cell_moments([&](int q) { return G[q].x; });
+            if (row | (ends & 8u)) m1 = cell_moments([&](int q) { return G[q].y; });
+            // halo rows of the pair; within the buffer, as every pulled row is
+            if (row & 4u) ghost_pair<1, 0>(G, m0, m1, out - rs);
+            if (row & 8u) ghost_pair<1, 1>(G, m0, m1, out + rs);
+            if (row & 16u) ghost_pair<2, 0>(G, m0, m1, out - ps);
+            if (row & 32u) ghost_pair<2, 1>(G, m0, m1, out + ps);
+            if (ends & 1u) ghost_end<0>(m0, 1.0f, fa, a.xf, L, j, k, [&](int q) { return G[q].x; });
+            if (ends & 10u)
+                ghost_end<1>(xhi0 ? m0 : m1, 1.0f, fa, a.xf, L, j, k, [&](int q) { return xhi0 ? G[q].x : G[q].y; });
+            if (fa.face_mom) keep_face_moments(fa, L, row, ends, c0, j, k, m0, m1);
+            return;
+        }
+    }
 
     if (xlo | xhi0 | xhi1)
     {
@@ -495,10 +633,49 @@ __host__ __device__ constexpr int ghost_slot(int q)
     return t[q];
 }
 
-template <int P, int WARPS, int MINB>
+// The next step's sources on a word of results: as stored, one source after another.
+__device__ __forceinline__ void add_sources(unsigned (&w)[Q], const SourceNext* __restrict__ nx, unsigned sources,
+                                            int c0, int j, int k, const Layout& L)
+{
+    while (sources)
+    {
+        const int s = __ffs(sources) - 1;
+        sources &= sources - 1;
+        const SourceBox b = nx->box[s];
+        const int row = ((k - b.k0) * b.n + (j - b.j0)) * b.n, d = c0 + 1 - b.i0;
+        const bool in0 = d >= 0 && d < b.n, in1 = d + 1 >= 0 && d + 1 < b.n && c0 + 1 < L.nx;
+        float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
+        if (in0) a0 = nx->add[s][row + d];
+        if (in1) a1 = nx->add[s][row + d + 1];
+        if (a0.w != 0.f)
+        {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) w[q] = set_lo(w[q], h2f(w[q]).x + source_gain(a0, q));
+        }
+        if (a1.w != 0.f)
+        {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) w[q] = set_hi(w[q], h2f(w[q]).y + source_gain(a1, q));
+        }
+    }
+}
+
+template <int AXIS, int SIDE>
+__device__ __forceinline__ void ghost_pair(const unsigned (&w)[Q], const float4& m0, const float4& m1, float inv_scale,
+                                           unsigned* ghost)
+{
+    float lo[Q];
+    nscbc<AXIS, SIDE>(m0, inv_scale, [&](int q) { return h2f(w[q]).x; }, [&](int q, float v) { lo[q] = v; });
+    nscbc<AXIS, SIDE>(m1, inv_scale, [&](int q) { return h2f(w[q]).y; },
+                      [&](int q, float v) { ghost[32 * q] = f2h(make_float2(lo[q], v)); });
+}
+
+// MODE: as k_step, the first `side` blocks beside the pipelines.
+template <int P, int WARPS, int MINB, int MODE>
 __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __restrict__ fin,
                                                                __half* __restrict__ fout, Layout L, StepArgs a,
-                                                               float inv_scale)
+                                                               float inv_scale, const __grid_constant__ FusedArgs fa,
+                                                               int side)
 {
     constexpr int S = P + 2;   // ring slots: blocks t - 1 .. t + P
     constexpr uint32_t kDirBits = (1u << Q) - 1u;
@@ -507,9 +684,18 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
     const int warp = threadIdx.x >> 5;
     unsigned char* ring = wp_smem + warp * (S * wp::kSlotBytes);
     const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
+    constexpr bool FUSED = MODE == kFused;
+    if constexpr (MODE != kPlain)
+    {
+        if ((int)blockIdx.x < side)
+        {
+            side_block<__half, MODE>(fin, L, a, fa, blockIdx.x, reinterpret_cast<double*>(wp_smem));
+            return;
+        }
+    }
     const int nrows = L.ny * L.nz;
-    const int all_warps = gridDim.x * WARPS;
-    const int r0 = blockIdx.x * WARPS + warp;   // rows r0, r0 + all_warps, ...; r = (k-1) ny + (j-1)
+    const int all_warps = ((int)gridDim.x - (MODE != kPlain ? side : 0)) * WARPS;
+    const int r0 = ((int)blockIdx.x - (MODE != kPlain ? side : 0)) * WARPS + warp;   // rows r0, r0 + all_warps, ...; r = (k-1) ny + (j-1)
     if (r0 >= nrows) return;
 
     // element offsets of this lane's five 16-byte pieces from the destination block
@@ -579,6 +765,9 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
     const unsigned* own = nullptr;   // this lane's word of line 0 of the block (line q: own[32 q])
     unsigned* outp = nullptr;
     float syz = 0.f;
+    // FUSED: what the row's results still take: bits 0-7 sources, bits 8-13 the open faces that the row or
+    // one of its ends borders, bit 14 the x-face exports of a step that leaves its results as they are
+    unsigned todo = 1u << 14;
     const auto cc_row = [&]() {
         cc_k = 1 + cc_r / L.ny;
         cc_j = 1 + cc_r - (cc_k - 1) * L.ny;
@@ -587,6 +776,14 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
         outp = reinterpret_cast<unsigned*>(fout + e) + lane;
         c0 = 2 * lane;
         syz = fmaxf(__ldg(a.sig_y + cc_j - 1), __ldg(a.sig_z + cc_k - 1));
+        if constexpr (FUSED)
+        {
+            if (fa.next->fill != 0)
+            {
+                todo = (row_faces(fa.open, cc_j, cc_k, L) | (fa.open & 3u)) << 8;
+                if (fa.src.nsrc > 0) todo |= sources_of_row(fa.next, fa.src.nsrc, lane, cc_j, cc_k);
+            }
+        }
     };
     const auto cc_next = [&]() {
         own += 19 * 32;
@@ -709,11 +906,12 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
         {
             const float2 sg = make_float2(fmaxf(sx0, syz), fmaxf(sx1, syz));
             collide2_grouped(w, inv_scale, a.omega, sg, (lk0 & kSolidSelfBit) != 0u, (lk1 & kSolidSelfBit) != 0u);
+            if (FUSED && (todo & 0xffu)) add_sources(w, fa.next, todo & 0xffu, c0, j, k, L);
 #pragma unroll
             for (int q = 0; q < Q; ++q)
                 if (LBM_IN(kChkHwStore, 2 * (outp - reinterpret_cast<unsigned*>(fout)) + 64 * q, L.total - 1))
                     outp[32 * q] = w[q];
-            if (edge && (xlo | xhi))
+            if ((todo & (1u << 14)) && edge && (xlo | xhi))
             {
 #pragma unroll
                 for (int q = 0; q < Q; ++q)
@@ -724,6 +922,27 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
                     if (xhi && last == 0) a.xf.xexp[a.xf.exp_index(1, q, j, k, L.ny, L.nz)] = h2f(w[q]).x;
                     if (xhi && last == 1) a.xf.xexp[a.xf.exp_index(1, q, j, k, L.ny, L.nz)] = h2f(w[q]).y;
                 }
+            }
+            if (FUSED && ((todo & (60u << 8)) || edge))
+            {
+                // from the values as stored; a row's end takes the moments of its own cell only, unless the
+                // whole row is a face
+                const unsigned row = (todo >> 8) & 60u, open = (todo >> 8) & 3u;
+                const unsigned ends = (xlo ? open & 1u : 0u) | (last == 0 ? open & 2u : 0u) |
+                                      (last == 1 ? (open & 2u) << 2 : 0u);
+                float4 m0 = make_float4(0.f, 0.f, 0.f, 0.f), m1 = m0;
+                if (row | (ends & 3u)) m0 = cell_moments([&](int q) { return h2f(w[q]).x; });
+                if (row | (ends & 8u)) m1 = cell_moments([&](int q) { return h2f(w[q]).y; });
+                const int rsw = (int)(L.row_stride >> 1), psw = (int)(L.plane_stride >> 1);
+                if (row & 4u) ghost_pair<1, 0>(w, m0, m1, inv_scale, outp - rsw);
+                if (row & 8u) ghost_pair<1, 1>(w, m0, m1, inv_scale, outp + rsw);
+                if (row & 16u) ghost_pair<2, 0>(w, m0, m1, inv_scale, outp - psw);
+                if (row & 32u) ghost_pair<2, 1>(w, m0, m1, inv_scale, outp + psw);
+                if (ends & 1u)
+                    ghost_end<0>(m0, inv_scale, fa, a.xf, L, j, k, [&](int q) { return h2f(w[q]).x; });
+                if (ends & 10u)
+                    ghost_end<1>(last == 0 ? m0 : m1, inv_scale, fa, a.xf, L, j, k,
+                                 [&](int q) { return last == 0 ? h2f(w[q]).x : h2f(w[q]).y; });
             }
         }
         __syncwarp();   // every lane is done with slot t - 1 before the next copy lands there
@@ -819,213 +1038,68 @@ __global__ void __launch_bounds__(128) k_build_links(const uint8_t* __restrict__
 }
 
 // ---------------------------------------------------------------- source
-__device__ double block_sum(double v, double* red)
-{
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) red[warp] = v;
-    __syncthreads();
-    double t = 0.0;
-    const int nw = (blockDim.x + 31) >> 5;
-    for (int w = 0; w < nw; ++w) t += red[w];
-    return t;
-}
-
-// Source injection (LBMSolver::apply_source 06:576-667): weights of the
-// (2R+1)^3 Gaussian stencil (or the 8 trilinear weights) are normalised over
-// the FLUID cells of the grid, A = mass / sum_w, and every FLUID cell gains
-// w_q * A * w_cell in each direction.  One block; sources run in order.
-// Cells next to the x faces also update their x-face export.
+// Source injection (LBMSolver::apply_source 06:576-667), block 0: every FLUID
+// cell of a source's stencil gains its amounts.  One block; sources run in order.
+// Cells next to the x faces also update their x-face export.  Block 1, at the
+// start of a batch of fused steps: the sources of the next step.
 template <typename S>
-__global__ void __launch_bounds__(512) k_source(S* __restrict__ f, Layout L, StepArgs sa, SourceArgs a)
+__global__ void __launch_bounds__(512) k_source(S* __restrict__ f, Layout L, StepArgs sa, SourceArgs a, int parity,
+                                                SourceNext* __restrict__ next)
 {
     __shared__ double red[32];
-    const int tid = threadIdx.x;
+    if (blockIdx.x == 1)
+    {
+        const long long s = a.ctl->step[parity];
+        prepare_sources(next, a, s + 1, s < a.ctl->last, L, sa.links, red);
+        return;
+    }
     for (int s = 0; s < a.nsrc; ++s)
     {
         SourceEntry e;
         if (a.ctl)
         {
-            const long long row = a.ctl->step - a.ctl->table_base;
+            const long long row = a.ctl->step[parity] - a.ctl->table_base;
             e = a.table[row * a.nsrc + s];
         }
         else
         {
             e = a.direct[s];
         }
-        if (e.mass == 0.0) continue;
-        const SourceStatic st = a.st[s];
-        int gi = 0, gj = 0, gk = 0;
-        bool in = false;
-        double ww = 0.0;
-        if (st.injection == 1)
-        {
-            const double fx = (e.cx - a.x_min) / a.dx - 0.5;
-            const double fy = (e.cy - a.y_min) / a.dx - 0.5;
-            const double fz = (e.cz - a.z_min) / a.dx - 0.5;
-            const int i0 = (int)floor(fx), j0 = (int)floor(fy), k0 = (int)floor(fz);
-            const double tx = fx - i0, ty = fy - j0, tz = fz - k0;
-            if (tid < 8)
-            {
-                gi = i0 + (tid & 1);
-                gj = j0 + ((tid >> 1) & 1);
-                gk = k0 + (tid >> 2);
-                ww = ((tid & 1) ? tx : 1.0 - tx) * (((tid >> 1) & 1) ? ty : 1.0 - ty) * ((tid >> 2) ? tz : 1.0 - tz);
-                in = true;
-            }
-        }
-        else
-        {
-            const int R = st.radius, n = 2 * R + 1;
-            const int ic = (int)floor((e.cx - a.x_min) / a.dx);
-            const int jc = (int)floor((e.cy - a.y_min) / a.dx);
-            const int kc = (int)floor((e.cz - a.z_min) / a.dx);
-            if (ic < -R || ic >= L.nx + R || jc < -R || jc >= L.ny + R || kc - a.k_off < -R ||
-                kc - a.k_off >= L.nz + R)
-                continue;
-            if (tid < n * n * n)
-            {
-                gi = ic + tid % n - R;
-                gj = jc + (tid / n) % n - R;
-                gk = kc + tid / (n * n) - R;
-                const double x = a.x_min + (gi + 0.5) * a.dx;
-                const double y = a.y_min + (gj + 0.5) * a.dx;
-                const double z = a.z_min + (gk + 0.5) * a.dx;
-                const double ddx = x - e.cx, ddy = y - e.cy, ddz = z - e.cz;
-                const double r2 = ddx * ddx + ddy * ddy + ddz * ddz;
-                ww = exp(-0.5 * r2 / st.sigma2);
-                in = true;
-            }
-        }
-        // weights in the coordinates of the whole grid; a z-slab holds layers k_off..
-        gk -= a.k_off;
-        bool fluid = false;
-        if (in && gi >= 0 && gi < L.nx && gj >= 0 && gj < L.ny && gk >= 0 && gk < L.nz)
-            fluid = (sa.links[L.cell(gi + 1, gj + 1, gk + 1)] & kSolidSelfBit) == 0u;
-        const double bsum = block_sum(fluid ? ww : 0.0, red);
-        const double sum = e.wsum > 0.0 ? e.wsum : bsum;   // a stencil across a z-slab cut
-        if (sum < 1e-30) continue;
-        const double A = e.mass / sum;
-        // (the bounds-checked build skips a cell whose 19 directions leave the buffer; no
-        // thread leaves the loop early, every thread reaches the barrier below)
-        if (fluid && LBM_IN(kChkSource, L.elem(18, gi + 1, gj + 1, gk + 1), L.total))
-        {
-            const double add = A * ww * (double)a.scale;
+        SourceBox b{};
+        source_stencil(e, a.st[s], a, L, sa.links, red, b, [&](int c, const float4& add) {
+            const int i = b.i0 + c % b.n, j = b.j0 + (c / b.n) % b.n, k = b.k0 + c / (b.n * b.n);
+            // (the bounds-checked build skips a cell whose 19 directions leave the buffer)
+            if (add.w == 0.f || !LBM_IN(kChkSource, L.elem(18, i, j, k), L.total)) return;
             // the 19 directions of one cell are 19 distinct elements: every load
             // first (one round trip), then the stores
-            S* p = f + L.elem(0, gi + 1, gj + 1, gk + 1);   // direction q at p + q * bc
+            S* p = f + L.elem(0, i, j, k);   // direction q at p + q * bc
             float v[Q];
 #pragma unroll
             for (int q = 0; q < Q; ++q) v[q] = Io<S>::ldw(p + q * L.bc);
 #pragma unroll
             for (int q = 0; q < Q; ++q)
             {
-                Io<S>::st(p + q * L.bc, v[q] + (float)(wd(q) * add));
-                if (gi == 0 || gi == L.nx - 1)
+                Io<S>::st(p + q * L.bc, v[q] + source_gain(add, q));
+                if (i == 1 || i == L.nx)
                 {
                     const float gs = Io<S>::ldw(p + q * L.bc);   // the stored value, as the step would export it
-                    if (gi == 0) sa.xf.xexp[sa.xf.exp_index(0, q, gj + 1, gk + 1, L.ny, L.nz)] = gs;
-                    if (gi == L.nx - 1) sa.xf.xexp[sa.xf.exp_index(1, q, gj + 1, gk + 1, L.ny, L.nz)] = gs;
+                    if (i == 1) sa.xf.xexp[sa.xf.exp_index(0, q, j, k, L.ny, L.nz)] = gs;
+                    if (i == L.nx) sa.xf.xexp[sa.xf.exp_index(1, q, j, k, L.ny, L.nz)] = gs;
                 }
             }
-        }
+        });
         __syncthreads();
     }
 }
 
 // ---------------------------------------------------------------- ghosts
-// Characteristic open boundary (exchange_halos 06:684-835, MPI size 1): the
-// ghost cell next to interior cell I gets
-//   f_B = feq(rho_B, u_B) + (f_I - feq(rho_I, u_I)),
-// where u_B keeps the tangential velocity of I, and the normal velocity and
-// pressure carry only the outgoing invariant (incoming invariant zero).  In
-// stored deviation units (Gs = scale * g):
-//   geq(rho', r, u) = w (rho' + r (3 c.u + (4.5 (c.u)^2 - 1.5 u^2) / scale)).
-
-//
-// Only the 5 directions that point from the ghost into the interior (e_axis =
-// +1 on the low side, -1 on the high side) are ever pulled from a ghost cell
-// (by the step, the probes, the field output, the slab messages and the
-// adjoint); the fill computes and stores those and leaves the other 14 of the
-// ghost cell as they are.
+// G: the populations of cell I in, its ghost's inward directions out
 template <int AXIS, int SIDE>
-__host__ __device__ constexpr bool inward(int q)
+__device__ __forceinline__ void ghost_values(float (&G)[Q], float inv_scale, float4* face_mom, long long t)
 {
-    return (AXIS == 0 ? ex(q) : AXIS == 1 ? ey(q) : ez(q)) == (SIDE ? -1 : 1);
-}
-
-template <int AXIS, int SIDE>
-__device__ __forceinline__ void nscbc(float (&G)[Q], float inv_scale)
-{
-    constexpr int axis = AXIS, side = SIDE;
-    float rho, jx, jy, jz;
-    moments(G, rho, jx, jy, jz);
-    float rI = fmaf(rho, inv_scale, 1.0f);
-    float ux, uy, uz;
-    if (rI > 1e-30f)
-    {
-        ux = jx / rI;
-        uy = jy / rI;
-        uz = jz / rI;
-    }
-    else
-    {
-        rI = 1.0f;
-        rho = 0.0f;
-        ux = uy = uz = 0.0f;
-    }
-    const float cs = (float)kCs, cs2 = (float)kCs2;
-    const float pI = cs2 * rho;
-    const float un = axis == 0 ? ux : (axis == 1 ? uy : uz);
-    float unB, pB;
-    if (side == 0)
-    {
-        const float Wm = un - pI / cs;   // Wp = 0 (06:694-698)
-        unB = 0.5f * Wm;
-        pB = -0.5f * cs * Wm;
-    }
-    else
-    {
-        const float Wp = un + pI / cs;   // Wm = 0 (06:721-725)
-        unB = 0.5f * Wp;
-        pB = 0.5f * cs * Wp;
-    }
-    const float rhoB = pB / cs2;
-    const float rB = fmaf(rhoB, inv_scale, 1.0f);
-    const float bx = axis == 0 ? unB : ux, by = axis == 1 ? unB : uy, bz = axis == 2 ? unB : uz;
-    // geq(B) - geq(I) = w_q (d0 + c.v + c^T M c), a quadratic form in
-    // c_q whose ten coefficients are taken once per cell
-    const float k45 = 4.5f * inv_scale;
-    const float d0 = (rhoB - rho) - 1.5f * inv_scale * (rB * (bx * bx + by * by + bz * bz) - rI * (ux * ux + uy * uy + uz * uz));
-    const float vx = 3.0f * (rB * bx - rI * ux), vy = 3.0f * (rB * by - rI * uy), vz = 3.0f * (rB * bz - rI * uz);
-    const float mxx = k45 * (rB * bx * bx - rI * ux * ux), myy = k45 * (rB * by * by - rI * uy * uy),
-                mzz = k45 * (rB * bz * bz - rI * uz * uz);
-    const float mxy = 2.0f * k45 * (rB * bx * by - rI * ux * uy), mxz = 2.0f * k45 * (rB * bx * bz - rI * ux * uz),
-                myz = 2.0f * k45 * (rB * by * bz - rI * uy * uz);
-#pragma unroll
-    for (int q = 0; q < Q; ++q)
-    {
-        if (!inward<AXIS, SIDE>(q)) continue;
-        float e = d0;
-        if (ex(q)) e += mxx;
-        if (ey(q)) e += myy;
-        if (ez(q)) e += mzz;
-        if (ex(q) * ey(q)) e += ex(q) * ey(q) * mxy;
-        if (ex(q) * ez(q)) e += ex(q) * ez(q) * mxz;
-        if (ey(q) * ez(q)) e += ey(q) * ez(q) * myz;
-        if (ex(q)) e += ex(q) * vx;
-        if (ey(q)) e += ey(q) * vy;
-        if (ez(q)) e += ez(q) * vz;
-        G[q] = fmaf(wf(q), e, G[q]);
-    }
-}
-
-__device__ __forceinline__ void store_moments(const float (&G)[Q], float4* out)
-{
-    float rho, jx, jy, jz;
-    moments(G, rho, jx, jy, jz);
-    *out = make_float4(rho, jx, jy, jz);
+    const float4 m = cell_moments([&](int q) { return G[q]; });
+    if (face_mom) face_mom[t] = m;
+    nscbc<AXIS, SIDE>(m, inv_scale, [&](int q) { return G[q]; }, [&](int q, float v) { G[q] = v; });
 }
 
 // One face cell (two x-adjacent ones in FP16 y and z faces) of face (AXIS, SIDE).
@@ -1045,8 +1119,7 @@ __device__ __forceinline__ void ghost_cell(S* __restrict__ f, const Layout& L, c
             return;
 #pragma unroll
         for (int q = 0; q < Q; ++q) G[q] = a.xf.xexp[a.xf.exp_index(SIDE, q, j, k, L.ny, L.nz)];
-        if (a.face_mom) store_moments(G, a.face_mom + t);
-        nscbc<AXIS, SIDE>(G, inv_scale);
+        ghost_values<AXIS, SIDE>(G, inv_scale, a.face_mom, t);
 #pragma unroll
         for (int q = 0; q < Q; ++q)
             if (inward<AXIS, SIDE>(q)) a.xf.xgh[a.xf.gh_index(SIDE, q, j, k, L.ny, L.nz)] = G[q];
@@ -1088,12 +1161,10 @@ __device__ __forceinline__ void ghost_cell(S* __restrict__ f, const Layout& L, c
             }
         }
         const long long cell = F.first + (long long)vp * F.nu + up;   // the face enumeration of one cell a thread
-        if (a.face_mom) store_moments(G, a.face_mom + cell);
-        nscbc<AXIS, SIDE>(G, inv_scale);
+        ghost_values<AXIS, SIDE>(G, inv_scale, a.face_mom, cell);
         if (two)
         {
-            if (a.face_mom) store_moments(G1, a.face_mom + cell + 1);
-            nscbc<AXIS, SIDE>(G1, inv_scale);
+            ghost_values<AXIS, SIDE>(G1, inv_scale, a.face_mom, cell + 1);
 #pragma unroll
             for (int q = 0; q < Q; ++q)
                 if (inward<AXIS, SIDE>(q)) *reinterpret_cast<__half2*>(B + q * BCH) = __floats2half2_rn(G[q], G1[q]);
@@ -1118,8 +1189,7 @@ __device__ __forceinline__ void ghost_cell(S* __restrict__ f, const Layout& L, c
         S* B = f + L.elem(0, ci, gj, gk);
 #pragma unroll
         for (int q = 0; q < Q; ++q) G[q] = Io<S>::ld(I + q * BC);
-        if (a.face_mom) store_moments(G, a.face_mom + t);
-        nscbc<AXIS, SIDE>(G, inv_scale);
+        ghost_values<AXIS, SIDE>(G, inv_scale, a.face_mom, t);
 #pragma unroll
         for (int q = 0; q < Q; ++q)
             if (inward<AXIS, SIDE>(q)) Io<S>::st(B + q * BC, G[q]);
@@ -1147,40 +1217,13 @@ __global__ void __launch_bounds__(128) k_ghost(S* __restrict__ f, Layout L, Ghos
 }
 
 // ---------------------------------------------------------------- probes
-// rho - 1 at each probe cell for the step whose pre-step buffer is `f`
-// (the value LBMSolver::run records, 06:1085-1092; SOLID cells read 0).
+// One step's probe record on its own (single calls), one warp per probe.
 template <typename S>
-__global__ void __launch_bounds__(256) k_probe(const S* __restrict__ f, Layout L, StepArgs sa, ProbeArgs a)
+__global__ void __launch_bounds__(128) k_probe(const S* __restrict__ f, Layout L, StepArgs sa, ProbeArgs a)
 {
-    const long long row = a.ctl ? a.ctl->step - a.ctl->probe_base : a.direct_row;
-    const float inv_scale = 1.0f / a.scale;
-    for (int p = threadIdx.x; p < a.n; p += blockDim.x)
-    {
-        const int i = a.ijk[3 * p], j = a.ijk[3 * p + 1], k = a.ijk[3 * p + 2];
-        double val;
-        if (i < 0)
-        {
-            val = __longlong_as_double(0x7ff8000000000000LL);
-        }
-        else
-        {
-            bool solid;
-            float G[Q];
-            pull_cell<S>(f, L, sa, i, j, k, G, solid);
-            float rho = 0.f;
-#pragma unroll
-            for (int q = 0; q < Q; ++q) rho += G[q];
-            const float rp = rho * inv_scale;
-            if (solid) val = 0.0;
-            else if (1.0f + rp <= 0.f) val = 1e-12 - 1.0;
-            else val = (double)rp;
-            a.energy[p] += val * val;
-            if (!isfinite(val)) *a.nonfinite = 1;
-        }
-        a.out[row * a.n + p] = val;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0 && a.ctl) a.ctl->step += 1;
+    const long long row = a.ctl ? a.ctl->step[a.parity] - a.ctl->probe_base : a.direct_row;
+    const int p = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (p < a.n) probe_warp<S>(f, L, sa.links, sa.xf.xgh, a, row, p, threadIdx.x & 31);
 }
 
 template <typename S>
@@ -1279,7 +1322,7 @@ dim3 row_grid(const Layout& L) { return dim3((unsigned)((L.nx + 127) / 128), (un
 // Warp-pipelined FP16 step: dynamic shared memory (one ring per warp) and a
 // grid of as many CTAs as the GPU holds at once (every warp then walks rows
 // all_warps apart).  The attribute and the occupancy are set up once per device.
-template <int P, int WARPS, int MINB>
+template <int P, int WARPS, int MINB, int MODE>
 cudaError_t hw_ctas(int* out)
 {
     constexpr int smem = WARPS * (P + 2) * wp::kSlotBytes;
@@ -1292,10 +1335,10 @@ cudaError_t hw_ctas(int* out)
     std::lock_guard<std::mutex> lock(mu);
     if (!ctas[dev])
     {
-        e = cudaFuncSetAttribute(k_step_hw<P, WARPS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const auto kernel = k_step_hw<P, WARPS, MINB, MODE>;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         int per_sm = 0, sms = 0;
-        if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step_hw<P, WARPS, MINB>, 32 * WARPS, smem);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * WARPS, smem);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return e;
         if (per_sm < 1) return cudaErrorInvalidConfiguration;
@@ -1305,29 +1348,35 @@ cudaError_t hw_ctas(int* out)
     return cudaSuccess;
 }
 
-template <int P, int WARPS, int MINB>
+template <int P, int WARPS, int MINB, int MODE>
 cudaError_t launch_hw(const __half* fin, __half* fout, const Layout& L, const StepArgs& a, float inv_scale,
-                      cudaStream_t stream)
+                      const FusedArgs& fa, cudaStream_t stream)
 {
     // the per-lane source offsets are 32-bit
     if (L.plane_stride + L.row_stride + 19 * 64 > 0x7fffffffLL) return cudaErrorInvalidValue;
     int ctas = 0;
-    const cudaError_t e = hw_ctas<P, WARPS, MINB>(&ctas);
+    const cudaError_t e = hw_ctas<P, WARPS, MINB, MODE>(&ctas);
     if (e != cudaSuccess) return e;
     const long long need = ((long long)L.ny * L.nz + WARPS - 1) / WARPS;
-    const int grid = (int)(need < ctas ? need : ctas);
-    k_step_hw<P, WARPS, MINB><<<grid, 32 * WARPS, WARPS * (P + 2) * wp::kSlotBytes, stream>>>(fin, fout, L, a, inv_scale);
+    const int side = MODE != kPlain ? side_blocks(fa.probe.n, WARPS) : 0;
+    const int grid = (int)(need < ctas ? need : ctas) + side;
+    k_step_hw<P, WARPS, MINB, MODE>
+        <<<grid, 32 * WARPS, WARPS * (P + 2) * wp::kSlotBytes, stream>>>(fin, fout, L, a, inv_scale, fa, side);
     return cudaGetLastError();
 }
 
-template <bool MOM>
+template <bool MOM, int MODE>
 cudaError_t launch_pair_step(const float* fin, float* fout, const Layout& L, const StepArgs& a, PairMoments* mom,
-                             cudaStream_t stream)
+                             const FusedArgs& fa, cudaStream_t stream)
 {
     const PairLaunch g = pair_launch(L);
-    if (g.bx == 4) k_step<float, 4, MOM><<<g.grid, kPairBlock, 0, stream>>>(fin, fout, L, a, 1.0f, mom);
-    else if (g.bx == 2) k_step<float, 2, MOM><<<g.grid, kPairBlock, 0, stream>>>(fin, fout, L, a, 1.0f, mom);
-    else k_step<float, 1, MOM><<<g.grid, kPairBlock, 0, stream>>>(fin, fout, L, a, 1.0f, mom);
+    dim3 grid = g.grid;
+    const int per_layer = (int)(grid.x * grid.y);
+    const int zx = MODE != kPlain ? (side_blocks(fa.probe.n, kPairBlock / 32) + per_layer - 1) / per_layer : 0;
+    grid.z += zx;
+    if (g.bx == 4) k_step<4, MOM, MODE><<<grid, kPairBlock, 0, stream>>>(fin, fout, L, a, mom, fa, zx);
+    else if (g.bx == 2) k_step<2, MOM, MODE><<<grid, kPairBlock, 0, stream>>>(fin, fout, L, a, mom, fa, zx);
+    else k_step<1, MOM, MODE><<<grid, kPairBlock, 0, stream>>>(fin, fout, L, a, mom, fa, zx);
     return cudaGetLastError();
 }
 
@@ -1386,27 +1435,46 @@ cudaError_t prepare_step(int storage)
 {
     if (storage == 0) return cudaSuccess;
     int ctas = 0;
-    return hw_ctas<2, 4, 5>(&ctas);
+    cudaError_t e = hw_ctas<2, 4, 5, kPlain>(&ctas);
+    if (e == cudaSuccess) e = hw_ctas<2, 4, 5, kSide>(&ctas);
+    return e != cudaSuccess ? e : hw_ctas<2, 4, 5, kFused>(&ctas);
 }
+
+namespace {
+template <int MODE>
+cudaError_t launch_step_mode(int storage, const void* fin, void* fout, const Layout& L, const StepArgs& a, float scale,
+                             const FusedArgs& fa, cudaStream_t stream)
+{
+    if (storage == 0) return launch_pair_step<false, MODE>((const float*)fin, (float*)fout, L, a, nullptr, fa, stream);
+    return launch_hw<2, 4, 5, MODE>((const __half*)fin, (__half*)fout, L, a, 1.0f / scale, fa, stream);
+}
+}  // namespace
 
 cudaError_t launch_step(int storage, const void* fin, void* fout, const Layout& L, const StepArgs& a,
                         float scale, cudaStream_t stream)
 {
-    if (storage == 0) return launch_pair_step<false>((const float*)fin, (float*)fout, L, a, nullptr, stream);
-    return launch_hw<2, 4, 5>((const __half*)fin, (__half*)fout, L, a, 1.0f / scale, stream);
+    return launch_step_mode<kPlain>(storage, fin, fout, L, a, scale, FusedArgs{}, stream);
+}
+
+cudaError_t launch_batched_step(int storage, const void* fin, void* fout, const Layout& L, const StepArgs& a,
+                                float scale, const FusedArgs& fa, bool fused, cudaStream_t stream)
+{
+    if (fused) return launch_step_mode<kFused>(storage, fin, fout, L, a, scale, fa, stream);
+    return launch_step_mode<kSide>(storage, fin, fout, L, a, scale, fa, stream);
 }
 
 cudaError_t launch_step_moments(const float* fin, float* fout, const Layout& L, const StepArgs& a,
                                 PairMoments* mom, cudaStream_t stream)
 {
-    return launch_pair_step<true>(fin, fout, L, a, mom, stream);
+    return launch_pair_step<true, kPlain>(fin, fout, L, a, mom, FusedArgs{}, stream);
 }
 
 cudaError_t launch_source(int storage, void* f, const Layout& L, const StepArgs& sa, const SourceArgs& a,
-                          cudaStream_t stream)
+                          int parity, SourceNext* next, cudaStream_t stream)
 {
-    if (storage == 0) k_source<float><<<1, 512, 0, stream>>>((float*)f, L, sa, a);
-    else k_source<__half><<<1, 512, 0, stream>>>((__half*)f, L, sa, a);
+    const unsigned blocks = next ? 2 : 1;
+    if (storage == 0) k_source<float><<<blocks, 512, 0, stream>>>((float*)f, L, sa, a, parity, next);
+    else k_source<__half><<<blocks, 512, 0, stream>>>((__half*)f, L, sa, a, parity, next);
     return cudaGetLastError();
 }
 
@@ -1422,8 +1490,10 @@ cudaError_t launch_ghost(int storage, void* f, const Layout& L, const GhostArgs&
 cudaError_t launch_probe(int storage, const void* f, const Layout& L, const StepArgs& sa, const ProbeArgs& a,
                          cudaStream_t stream)
 {
-    if (storage == 0) k_probe<float><<<1, 256, 0, stream>>>((const float*)f, L, sa, a);
-    else k_probe<__half><<<1, 256, 0, stream>>>((const __half*)f, L, sa, a);
+    if (a.n <= 0) return cudaSuccess;
+    const unsigned blocks = (unsigned)((a.n + 3) / 4);
+    if (storage == 0) k_probe<float><<<blocks, 128, 0, stream>>>((const float*)f, L, sa, a);
+    else k_probe<__half><<<blocks, 128, 0, stream>>>((const __half*)f, L, sa, a);
     return cudaGetLastError();
 }
 

@@ -34,7 +34,7 @@ __device__ __forceinline__ uint32_t near_bits(const StepArgs& a, const Layout& L
 __device__ __forceinline__ float field_mass(const SchemeAArgs& b, int ahead)
 {
     if (!b.ctl) return b.mass_direct[ahead];
-    const long long row = b.ctl->step - b.ctl->table_base + ahead;
+    const long long row = b.ctl->step[b.parity] - b.ctl->table_base + ahead;
     return (float)b.table[row * b.nsrc + b.src_index].mass;
 }
 
@@ -715,7 +715,7 @@ __global__ void __launch_bounds__(128) k_set_density_a(float* __restrict__ f, fl
 __global__ void __launch_bounds__(256) k_probe_a(const float* __restrict__ f, Layout L, StepArgs sa, SchemeAArgs b,
                                                  ProbeArgs a)
 {
-    const long long row = a.ctl ? a.ctl->step - a.ctl->probe_base : a.direct_row;
+    const long long row = a.ctl ? a.ctl->step[a.parity] - a.ctl->probe_base : a.direct_row;
     for (int p = threadIdx.x; p < a.n; p += blockDim.x)
     {
         const int i = a.ijk[3 * p], j = a.ijk[3 * p + 1], k = a.ijk[3 * p + 2];
@@ -739,7 +739,7 @@ __global__ void __launch_bounds__(256) k_probe_a(const float* __restrict__ f, La
         a.out[row * a.n + p] = val;
     }
     __syncthreads();
-    if (threadIdx.x == 0 && a.ctl) a.ctl->step += 1;
+    if (threadIdx.x == 0 && a.ctl) a.ctl->step[a.parity ^ 1] = a.ctl->step[a.parity] + 1;
 }
 
 __global__ void __launch_bounds__(128) k_field_rho_a(const float* __restrict__ f, float* __restrict__ out, Layout L,

@@ -60,3 +60,36 @@ def test_step_matches_oracle(size, storage, gpu):
         dg, do = (s.get_f().reshape(nz, ny, nx, 19)[1:-1, 1:-1, 1:-1] - w for s in (g, o))
         assert np.max(np.abs(dg - do)) <= FP32_STATE_TOL * np.max(np.abs(do))
     g.close()
+
+
+@pytest.mark.parametrize("size", [(33, 10, 8), (65, 13, 6), (128, 10, 9), (191, 7, 8)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("storage", [abi.LBM_STORE_F32, abi.LBM_STORE_F16], ids=["f32", "f16"])
+@pytest.mark.parametrize("split", [(13,), (1, 1, 1, 2, 1, 7), (2, 11), (5, 8)], ids=str)
+def test_batches_equal_single_calls(size, storage, split, gpu):
+    """However a run is split into batches, every batched step (which applies the next step's sources and
+    ghosts to its own results) gives the bits of the single calls, sources against the open faces included."""
+    cfg, srcs, probes, tris = case(size, storage, ground=True)
+    a = nlos_lbm.Solver(cfg, srcs, probes, triangles=tris)
+    b = nlos_lbm.Solver(cfg, srcs, probes, triangles=tris)
+    for s in range(sum(split)):
+        a.apply_source(s * a.dt)
+        a.exchange_halos()
+        a.step_collision_bgk()
+        a.record_probes()
+    for n in split:
+        b.step(n)
+    assert np.array_equal(a.get_probes(), b.get_probes())
+    assert np.array_equal(a.get_probe_energy(), b.get_probe_energy())
+    assert np.array_equal(a.get_f(), b.get_f())
+    assert np.array_equal(a.get_rho(), b.get_rho())
+    # single calls after a batch, and a batch after single calls
+    for s in range(sum(split), sum(split) + 2):
+        b.apply_source(s * b.dt)
+        b.exchange_halos()
+        b.step_collision_bgk()
+        b.record_probes()
+    a.step(2)
+    assert np.array_equal(a.get_f(), b.get_f())
+    assert np.array_equal(a.get_probes(), b.get_probes())
+    a.close()
+    b.close()
