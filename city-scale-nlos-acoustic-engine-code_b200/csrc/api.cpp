@@ -1226,7 +1226,9 @@ cudaError_t timed_step_launch(lbm_handle* h, int parity, bool batched, long long
         StepArgs sa;
         SchemeAArgs b;
         scheme_a_args(h, parity, batched, s, sa, b);
-        return launch_step_a((const float*)h->f[parity], (float*)h->f[parity ^ 1], h->L, sa, b, h->stream);
+        ProbeArgs pr{};
+        if (batched) pr = probe_args(h, true, 0, parity);
+        return launch_step_a((const float*)h->f[parity], (float*)h->f[parity ^ 1], h->L, sa, b, pr, h->stream);
     };
     cudaError_t e;
     if (h->timing)
@@ -1296,26 +1298,7 @@ cudaError_t enqueue_batched_step(lbm_handle* h, int parity, int& kernels)
     cudaError_t e = cudaSuccess;
     void* fc = h->f[parity];
     kernels = 0;
-    if (h->scheme_a())
-    {
-        // the field source acts inside the step; halo copies and probes read the same buffer
-        StepArgs sa;
-        SchemeAArgs b;
-        scheme_a_args(h, parity, true, 0, sa, b);
-        e = timed_step_launch(h, parity, true, 0);
-        if (e != cudaSuccess) return e;
-        kernels++;
-        if (b.copy)
-        {
-            e = launch_copy_a((const float*)fc, (float*)h->f[parity ^ 1], h->L, sa, b, h->stream);
-            if (e != cudaSuccess) return e;
-            kernels++;
-        }
-        e = launch_probe_a((const float*)fc, h->L, sa, b, probe_args(h, true, 0, parity), h->stream);
-        kernels++;
-        return e;
-    }
-    if (!fused_steps(h))
+    if (!h->scheme_a() && !fused_steps(h))
     {
         const StepArgs sa = h->step_args(parity);
         if (!h->srcs.empty())
@@ -1333,6 +1316,16 @@ cudaError_t enqueue_batched_step(lbm_handle* h, int parity, int& kernels)
     }
     if (e == cudaSuccess) e = timed_step_launch(h, parity, true, 0);
     kernels++;
+    if (e == cudaSuccess && h->scheme_a())
+    {
+        StepArgs sa;
+        SchemeAArgs b;
+        scheme_a_args(h, parity, true, 0, sa, b);
+        if (step_a_has_side(b)) return e;
+        e = launch_side_a((const float*)fc, (float*)h->f[parity ^ 1], h->L, sa, b, probe_args(h, true, 0, parity),
+                          h->stream);
+        kernels++;
+    }
     return e;
 }
 
@@ -1588,12 +1581,13 @@ extern "C" int lbm_step_collision_bgk(lbm_handle* h)
     CK(cudaSetDevice(h->device), "cudaSetDevice");
     CK(timed_step_launch(h, h->cur, false, h->step), "step kernel");
     h->launches++;
-    if (h->scheme_a() && h->aa.copy)
+    if (h->scheme_a() && h->aa.copy && !step_a_has_side(h->aa))
     {
         StepArgs sa;
         SchemeAArgs b;
         scheme_a_args(h, h->cur, false, h->step, sa, b);
-        CK(launch_copy_a((const float*)h->f[h->cur], (float*)h->f[h->cur ^ 1], h->L, sa, b, h->stream), "halo copy");
+        CK(launch_side_a((const float*)h->f[h->cur], (float*)h->f[h->cur ^ 1], h->L, sa, b, ProbeArgs{}, h->stream),
+           "halo copy");
         h->launches++;
     }
     h->xgh_last = h->cur;

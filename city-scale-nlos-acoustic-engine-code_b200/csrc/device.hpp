@@ -211,7 +211,7 @@ struct FusedArgs
 // of the opposite direction: each fluid cell writes that value into the
 // SOLID neighbour's (otherwise unused) slot for the next step, so the next
 // pull reads it like any other.  Zero-gradient halos are collided copies of
-// the nearest interior cell, written for the next step by k_copy_a.  x-halo
+// the nearest interior cell, written for the next step beside the step.  x-halo
 // values live in two x-face arrays that alternate with the step parity.
 struct SchemeAArgs
 {
@@ -235,7 +235,7 @@ struct SchemeAArgs
     int parity;                // step counter ctl->step[parity]
     float mass_direct[2];      // mass of step s and of step s + 1 (direct launches)
     float* xgh_out;            // x-halo values written for the next step
-    int copy;                  // zero-gradient halos on every face
+    int copy;                  // zero-gradient halos on every face (copies written by the step's launch)
     const float* sg_x;         // destination blend toward rest (01:207-225, 01:343-347): strength per
     const float* sg_y;         //   interior column i-1, likewise sg_y, sg_z; a cell's is the maximum
     const float* sg_z;         //   of the three, 0 outside the layer
@@ -339,12 +339,15 @@ cudaError_t launch_export_f(int storage, const void* f, double* out, const Layou
 cudaError_t launch_import_f(int storage, void* f, const double* in, const Layout& L, const XFace& xf, float scale,
                             cudaStream_t stream);
 
-// Scheme A: fused step (FP32 storage), the zero-gradient halo copies of the
-// next step, the initial state, and probes / field of a scheme-A state.
+// Scheme A: fused step (FP32 storage) with the zero-gradient halo copies of the
+// next step and, where probe.ctl is set (batched steps), the probe record and the step counter; the initial state, and probes / field of a scheme-A state.
 cudaError_t launch_step_a(const float* fin, float* fout, const Layout& L, const StepArgs& a, const SchemeAArgs& b,
-                          cudaStream_t stream);
-cudaError_t launch_copy_a(const float* fin, float* fout, const Layout& L, const StepArgs& a, const SchemeAArgs& b,
-                          cudaStream_t stream);
+                          const ProbeArgs& probe, cudaStream_t stream);
+// Whether launch_step_a's launch holds the halo copies, probes and counter; else launch_side_a follows it
+// (after a single call only where there are copies).
+inline bool step_a_has_side(const SchemeAArgs& b) { return !(b.field_mode == 2 || b.sg_xy || b.fld_xy); }
+cudaError_t launch_side_a(const float* fin, float* fout, const Layout& L, const StepArgs& a, const SchemeAArgs& b,
+                          const ProbeArgs& probe, cudaStream_t stream);
 cudaError_t launch_init_a(float* f0, float* f1, float* xgh0, float* xgh1, const uint8_t* mask_ref, const Layout& L,
                           const SchemeAArgs& b, cudaStream_t stream);
 cudaError_t launch_probe_a(const float* f, const Layout& L, const StepArgs& sa, const SchemeAArgs& b,

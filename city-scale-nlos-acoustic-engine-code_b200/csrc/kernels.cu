@@ -332,24 +332,27 @@ __device__ __forceinline__ PairMoments pack_moments(float4 m0, float4 m1)
                         (v5 >> 4) | (v6 << 8) | (v7 << 20)}};
 }
 
-// MODE: the first zx layers of blocks are the blocks beside the step; a fused
+// MODE: the last side_rows rows of blocks of every layer are the blocks beside
+// the step (a block's own row and plane stay plain block indices); a fused
 // step writes the x-face exports only where its results stay as they are.
 // 80 registers (24 warps per SM) for the fused step: at the plain step's 72 it
 // spills 40 bytes, 256x256x128 233 us a step against 218; at 96 250 us.
 template <int BX, bool MOM, int MODE>
 __global__ void __launch_bounds__(kPairBlock, MODE == kFused ? 6 : 0) k_step(const float* __restrict__ fin, float* __restrict__ fout, Layout L,
                                                       StepArgs a, PairMoments* __restrict__ mom,
-                                                      const __grid_constant__ FusedArgs fa, int zx)
+                                                      const __grid_constant__ FusedArgs fa, int side_rows)
 {
     using S = float;
     using P = PairIo<S>;
     constexpr bool FUSED = MODE == kFused;
     if constexpr (MODE != kPlain)
     {
-        if ((int)blockIdx.z < zx)
+        const int row0 = (int)gridDim.y - side_rows;
+        if ((int)blockIdx.y >= row0)
         {
             __shared__ double red[16];
-            const int block = (int)((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
+            const int block =
+                ((int)blockIdx.z * side_rows + (int)blockIdx.y - row0) * (int)gridDim.x + (int)blockIdx.x;
             if (block < side_blocks(fa.probe.n, kPairBlock / 32)) side_block<S, MODE>(fin, L, a, fa, block, red);
             return;
         }
@@ -361,7 +364,7 @@ __global__ void __launch_bounds__(kPairBlock, MODE == kFused ? 6 : 0) k_step(con
     const bool active = c0r < L.nx;
     const int c0 = active ? c0r : ((L.nx - 1) & ~1);         // inactive lanes shadow a valid pair
     const int j = pair_row<BX>();
-    const int k = (int)blockIdx.z - (MODE != kPlain ? zx : 0) + 1;
+    const int k = blockIdx.z + 1;
     if (BX < 4 && j > L.ny) return;   // whole warps
     const long long e0 = L.elem(0, c0 + 1, j, k);
     const S* own = fin + e0;
@@ -1371,12 +1374,12 @@ cudaError_t launch_pair_step(const float* fin, float* fout, const Layout& L, con
 {
     const PairLaunch g = pair_launch(L);
     dim3 grid = g.grid;
-    const int per_layer = (int)(grid.x * grid.y);
-    const int zx = MODE != kPlain ? (side_blocks(fa.probe.n, kPairBlock / 32) + per_layer - 1) / per_layer : 0;
-    grid.z += zx;
-    if (g.bx == 4) k_step<4, MOM, MODE><<<grid, kPairBlock, 0, stream>>>(fin, fout, L, a, mom, fa, zx);
-    else if (g.bx == 2) k_step<2, MOM, MODE><<<grid, kPairBlock, 0, stream>>>(fin, fout, L, a, mom, fa, zx);
-    else k_step<1, MOM, MODE><<<grid, kPairBlock, 0, stream>>>(fin, fout, L, a, mom, fa, zx);
+    const int per_row = (int)(grid.x * grid.z);
+    const int side = MODE != kPlain ? (side_blocks(fa.probe.n, kPairBlock / 32) + per_row - 1) / per_row : 0;
+    grid.y += side;
+    if (g.bx == 4) k_step<4, MOM, MODE><<<grid, kPairBlock, 0, stream>>>(fin, fout, L, a, mom, fa, side);
+    else if (g.bx == 2) k_step<2, MOM, MODE><<<grid, kPairBlock, 0, stream>>>(fin, fout, L, a, mom, fa, side);
+    else k_step<1, MOM, MODE><<<grid, kPairBlock, 0, stream>>>(fin, fout, L, a, mom, fa, side);
     return cudaGetLastError();
 }
 

@@ -9,6 +9,7 @@
 
 #include "check.cuh"
 #include "device.hpp"
+#include "epilogue.cuh"
 #include "lattice.cuh"
 
 namespace lbm {
@@ -160,7 +161,7 @@ struct ColumnValues
     float mass0, mass1;   // source mass of this step and of the next
 };
 
-template <int FEAT>
+template <int FEAT, bool SIDE>
 __device__ __forceinline__ void step_a_pair(const float* __restrict__ fin, float* __restrict__ fout, const Layout& L,
                                             const StepArgs& a, const SchemeAArgs& b, const ColumnValues& z,
                                             int lane, bool active, bool has1, int c0, int j, int k)
@@ -296,6 +297,9 @@ __device__ __forceinline__ void step_a_pair(const float* __restrict__ fin, float
                 const bool sol = c ? solid1 : solid0;
                 if (sol || !((lkc >> q) & 1u)) continue;
                 const int si = c0 + 1 + c - ex(q), sj = j - ey(q), sk = k - ez(q);
+                // zero-gradient halo cells hold copies, SOLID or not (side_block_a writes them in this launch)
+                if (SIDE && b.copy && (si == 0 || si == L.nx + 1 || sj == 0 || sj == L.ny + 1 || sk == 0 || sk == L.nz + 1))
+                    continue;
                 const float v = c ? G[inv(q)].y : G[inv(q)].x;
                 if (si == 0 || si == L.nx + 1) b.xgh_out[a.xf.gh_index(si == 0 ? 0 : 1, q, sj, sk, L.ny, L.nz)] = v;
                 else if (LBM_IN(kChkAStore, L.elem(q, si, sj, sk), L.total)) fout[L.elem(q, si, sj, sk)] = v;
@@ -465,10 +469,177 @@ __device__ __forceinline__ void step_a_pair(const float* __restrict__ fin, float
     }
 }
 
-template <int BLOCK, int MINB, int FEAT, int KZ>
-__global__ void __launch_bounds__(BLOCK, MINB) k_step_a(const float* __restrict__ fin, float* __restrict__ fout,
-                                                        Layout L, StepArgs a, SchemeAArgs b)
+// ---------------------------------------------------------------- halo copies
+// Zero-gradient halos (03:175-237): every halo cell is a copy of the nearest
+// interior cell I taken before the step and then collided like any cell,
+// with the halo's own tau (outside every ramp) and source weight.  For the
+// step after this one, the halo's post-collision values are
+// C_bulk(f(I)) + force(halo), with f(I) the populations arriving at I in this
+// step.  One thread per halo cell.  Every layer of blocks takes the ring of
+// halo cells of its own plane, whose sources the step's blocks of that layer
+// read at the same time (from L2 then: a value of an x-halo cell is a line of
+// its own), and a share of the two z-halo planes.
+struct HaloLayer
 {
+    int ring, share;   // cells of one plane's ring, and of the z-halo planes per layer
+};
+HaloLayer halo_layer(const Layout& L)
+{
+    const long long caps = 2LL * (L.nx + 2) * (L.ny + 2);
+    return HaloLayer{2 * (L.ny + 2) + 2 * L.nx, (int)((caps + L.nz - 1) / L.nz)};
+}
+__device__ __forceinline__ void copy_halo_cell(const float* __restrict__ fin, float* __restrict__ fout, const Layout& L,
+                                               const StepArgs& a, const SchemeAArgs& b, const HaloLayer& h, int layer,
+                                               int t)
+{
+    int ih, jh, kh;
+    if (t < h.ring)
+    {
+        kh = layer + 1;
+        const int nyt = L.ny + 2;
+        if (t < 2 * nyt)
+        {
+            ih = t < nyt ? 0 : L.nx + 1;
+            jh = t < nyt ? t : t - nyt;
+        }
+        else
+        {
+            const int u = t - 2 * nyt;
+            jh = u < L.nx ? 0 : L.ny + 1;
+            ih = 1 + (u < L.nx ? u : u - L.nx);
+        }
+    }
+    else
+    {
+        // 32-bit: launch_step_a rejects planes of 2^30 cells or more
+        const int plane = (L.nx + 2) * (L.ny + 2);
+        int u = layer * h.share + (t - h.ring);
+        if (t - h.ring >= h.share || u >= 2 * plane) return;
+        kh = u < plane ? 0 : L.nz + 1;
+        if (u >= plane) u -= plane;
+        jh = u / (L.nx + 2);
+        ih = u - jh * (L.nx + 2);
+    }
+    const int i = min(max(ih, 1), L.nx), j = min(max(jh, 1), L.ny), k = min(max(kh, 1), L.nz);
+    float G[Q];
+    uint32_t lk;
+    pull_a(fin, L, a, b, i, j, k, G, lk);
+    collide1(G, b.om_bulk, b);
+    if (b.field_mode == 1)
+    {
+        const float s = field_mass(b, 1) * field_weight(b, ih, jh, kh);
+#pragma unroll
+        for (int q = 0; q < Q; ++q) G[q] += force_term(b, q, s, b.om_bulk);
+    }
+    if (ih == 0 || ih == L.nx + 1)
+    {
+#pragma unroll
+        for (int q = 0; q < Q; ++q) b.xgh_out[a.xf.gh_index(ih == 0 ? 0 : 1, q, jh, kh, L.ny, L.nz)] = G[q];
+    }
+    else
+    {
+        float* out = fout + L.elem(0, ih, jh, kh);
+#pragma unroll
+        for (int q = 0; q < Q; ++q) out[q * BC] = G[q];
+    }
+}
+
+// ---------------------------------------------------------------- blocks beside the step
+// rho - 1 at probe p after the step that reads f (the reference records rho of
+// the arriving populations, 02:411, 03:438; SOLID cells read 0): one warp, lane
+// q takes direction q as pull_a does, the sum is taken in direction order.
+__device__ __forceinline__ void probe_warp_a(const float* __restrict__ f, const Layout& L, const StepArgs& sa,
+                                             const SchemeAArgs& b, const ProbeArgs& a, long long row, int p, int lane)
+{
+    const int i = a.ijk[3 * p], j = a.ijk[3 * p + 1], k = a.ijk[3 * p + 2];
+    if (i < 0)
+    {
+        if (lane == 0) record_probe(a, row, p, false, __longlong_as_double(0x7ff8000000000000LL));
+        return;
+    }
+    const uint32_t lk = sa.links[L.cell(i, j, k)];
+    float g = 0.f;
+    if (lane < Q)
+    {
+        const int q = lane, si = i - e_of<0>(q), sj = j - e_of<1>(q), sk = k - e_of<2>(q);
+        if (si == 0 || si == L.nx + 1) g = sa.xf.xgh[sa.xf.gh_index(si == 0 ? 0 : 1, q, sj, sk, L.ny, L.nz)];
+        else if (LBM_IN(kChkProbe, L.elem(q, si, sj, sk), L.total)) g = __ldg(f + L.elem(q, si, sj, sk));
+        if (!((lk >> q) & 1u))
+        {
+            if (b.field_mode == 0)
+                g = fmaf(q == 0 ? wf(0) : (q < 7 ? wf(1) : wf(7)), field_mass(b, 0) * field_weight(b, i, j, k), g);
+            if (b.blend)
+            {
+                const float sg = cell_blend(b, i, j, k);
+                g = fmaf(1.0f - sg, g, -sg * b.base[q]);
+            }
+        }
+    }
+    const float rho = sum_directions(g);
+    if (lane == 0) record_probe(a, row, p, true, (lk & kSolidSelfBit) ? 0.0 : (double)rho);
+}
+
+// Blocks beside a layer of the step: the halo copies of its plane, then a share
+// of the probe blocks of the launch, of which the first advances the step
+// counter (batched steps) and the others record a probe per warp.
+struct SideBlocks
+{
+    int rows;          // rows of blocks beside the step in every layer
+    int copy, probe;   // blocks of either kind per layer
+    HaloLayer halo;
+};
+SideBlocks side_blocks_a(const Layout& L, int gx, int copy, int nprobe)
+{
+    const HaloLayer h = halo_layer(L);
+    const int nc = copy ? (h.ring + h.share + kPairBlock - 1) / kPairBlock : 0;
+    const int np = (1 + (nprobe + 3) / 4 + L.nz - 1) / L.nz;
+    return SideBlocks{(nc + np + gx - 1) / gx, nc, np, h};
+}
+__device__ __forceinline__ void side_block_a(const float* __restrict__ fin, float* __restrict__ fout, const Layout& L,
+                                             const StepArgs& a, const SchemeAArgs& b, const ProbeArgs& pr,
+                                             const SideBlocks& n, int layer, int block)
+{
+    if (block < n.copy)
+    {
+        copy_halo_cell(fin, fout, L, a, b, n.halo, layer, block * kPairBlock + (int)threadIdx.x);
+        return;
+    }
+    if (block >= n.copy + n.probe || !pr.ctl) return;
+    const int pb = layer * n.probe + block - n.copy;
+    const long long s = pr.ctl->step[pr.parity];
+    if (pb == 0)
+    {
+        if (threadIdx.x == 0) pr.ctl->step[pr.parity ^ 1] = s + 1;
+        return;
+    }
+    const int p = (pb - 1) * 4 + (int)(threadIdx.x >> 5);
+    if (p < pr.n) probe_warp_a(fin, L, a, b, pr, s - pr.ctl->probe_base, p, threadIdx.x & 31);
+}
+
+// The blocks beside the step are the last side.rows rows of blocks of every
+// layer, so a block's own row and plane stay plain block indices (as layers of
+// their own they cost the instances 28-108 bytes of spills at their cap) and
+// the halo copies, which gather one line per value, run beside the blocks that
+// read the same lines: a 200x200x300 Doppler step 376 us with the copies and
+// the probes as launches of their own, 358 us with the copies spread over the
+// launch in any order, 334 us by plane.  SIDE = false (04's instance): they
+// are a launch of their own, k_side_a; in the instance they double its spills
+// (305 us against 267 on 04's grid).
+template <int BLOCK, int MINB, int FEAT, int KZ, bool SIDE>
+__global__ void __launch_bounds__(BLOCK, MINB) k_step_a(const float* __restrict__ fin, float* __restrict__ fout,
+                                                        Layout L, StepArgs a, SchemeAArgs b,
+                                                        const __grid_constant__ ProbeArgs pr, SideBlocks side)
+{
+    if constexpr (SIDE)
+    {
+        const int row0 = (int)gridDim.y - side.rows;
+        if ((int)blockIdx.y >= row0)
+        {
+            side_block_a(fin, fout, L, a, b, pr, side, blockIdx.z,
+                         ((int)blockIdx.y - row0) * (int)gridDim.x + (int)blockIdx.x);
+            return;
+        }
+    }
     const int lane = threadIdx.x & 31;
     const int c0r = 2 * (blockIdx.x * BLOCK + threadIdx.x);
     const bool active = c0r < L.nx;
@@ -477,7 +648,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_step_a(const float* __restrict_
     const int j = blockIdx.y + 1;
     if constexpr (FEAT < 2)
     {
-        step_a_pair<FEAT>(fin, fout, L, a, b, ColumnValues{}, lane, active, has1, c0, j, blockIdx.z + 1);
+        step_a_pair<FEAT, SIDE>(fin, fout, L, a, b, ColumnValues{}, lane, active, has1, c0, j, blockIdx.z + 1);
     }
     else
     {
@@ -519,75 +690,16 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_step_a(const float* __restrict_
         {
             const int k = k0 + kk;
             if (k > L.nz) break;
-            step_a_pair<FEAT>(fin, fout, L, a, b, z, lane, active, has1, c0, j, k);
+            step_a_pair<FEAT, SIDE>(fin, fout, L, a, b, z, lane, active, has1, c0, j, k);
         }
     }
 }
 
-// ---------------------------------------------------------------- halo copies
-// Zero-gradient halos (03:175-237): every halo cell is a copy of the nearest
-// interior cell I taken before the step and then collided like any cell,
-// with the halo's own tau (outside every ramp) and source weight.  For the
-// step after this one, the halo's post-collision values are
-// C_bulk(f(I)) + force(halo), with f(I) the populations arriving at I in this
-// step.  One thread per halo cell: x-halo planes (edges and corners
-// included), then the y-halo rows, then the z-halo rows.
-__global__ void __launch_bounds__(128) k_copy_a(const float* __restrict__ fin, float* __restrict__ fout, Layout L,
-                                                 StepArgs a, SchemeAArgs b)
+// The blocks beside the step as a launch of their own.
+__global__ void __launch_bounds__(kPairBlock) k_side_a(const float* __restrict__ fin, float* __restrict__ fout, Layout L,
+                                                       StepArgs a, SchemeAArgs b, ProbeArgs pr, SideBlocks side)
 {
-    // 32-bit index arithmetic: launch_copy_a rejects grids with 2^31 halo cells or more
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nyt = L.ny + 2, nzt = L.nz + 2;
-    const int pX = nyt * nzt, pY = L.nx * nzt, pZ = L.nx * L.ny;   // cells of one face
-    int ih, jh, kh;
-    if (t < 2 * pX)
-    {
-        const int r = t < pX ? t : t - pX;
-        ih = t < pX ? 0 : L.nx + 1;
-        kh = r / nyt;
-        jh = r - kh * nyt;
-    }
-    else if (t < 2 * pX + 2 * pY)
-    {
-        const int u = t - 2 * pX, r = u < pY ? u : u - pY;
-        jh = u < pY ? 0 : L.ny + 1;
-        kh = r / L.nx;
-        ih = 1 + r - kh * L.nx;
-    }
-    else if (t < 2 * pX + 2 * pY + 2 * pZ)
-    {
-        const int u = t - 2 * pX - 2 * pY, r = u < pZ ? u : u - pZ;
-        kh = u < pZ ? 0 : L.nz + 1;
-        const int jr = r / L.nx;
-        ih = 1 + r - jr * L.nx;
-        jh = 1 + jr;
-    }
-    else
-    {
-        return;
-    }
-    const int i = min(max(ih, 1), L.nx), j = min(max(jh, 1), L.ny), k = min(max(kh, 1), L.nz);
-    float G[Q];
-    uint32_t lk;
-    pull_a(fin, L, a, b, i, j, k, G, lk);
-    collide1(G, b.om_bulk, b);
-    if (b.field_mode == 1)
-    {
-        const float s = field_mass(b, 1) * field_weight(b, ih, jh, kh);
-#pragma unroll
-        for (int q = 0; q < Q; ++q) G[q] += force_term(b, q, s, b.om_bulk);
-    }
-    if (ih == 0 || ih == L.nx + 1)
-    {
-#pragma unroll
-        for (int q = 0; q < Q; ++q) b.xgh_out[a.xf.gh_index(ih == 0 ? 0 : 1, q, jh, kh, L.ny, L.nz)] = G[q];
-    }
-    else
-    {
-        float* out = fout + L.elem(0, ih, jh, kh);
-#pragma unroll
-        for (int q = 0; q < Q; ++q) out[q * BC] = G[q];
-    }
+    side_block_a(fin, fout, L, a, b, pr, side, blockIdx.y, blockIdx.x);
 }
 
 // ---------------------------------------------------------------- set-up
@@ -710,36 +822,12 @@ __global__ void __launch_bounds__(128) k_set_density_a(float* __restrict__ f, fl
 }
 
 // ---------------------------------------------------------------- probes, field
-// rho - 1 after the step that reads f (the reference records rho of the
-// arriving populations, 02:411, 03:438); SOLID cells read 0.
-__global__ void __launch_bounds__(256) k_probe_a(const float* __restrict__ f, Layout L, StepArgs sa, SchemeAArgs b,
+// One step's probe record on its own (single calls), one warp per probe.
+__global__ void __launch_bounds__(128) k_probe_a(const float* __restrict__ f, Layout L, StepArgs sa, SchemeAArgs b,
                                                  ProbeArgs a)
 {
-    const long long row = a.ctl ? a.ctl->step[a.parity] - a.ctl->probe_base : a.direct_row;
-    for (int p = threadIdx.x; p < a.n; p += blockDim.x)
-    {
-        const int i = a.ijk[3 * p], j = a.ijk[3 * p + 1], k = a.ijk[3 * p + 2];
-        double val;
-        if (i < 0)
-        {
-            val = __longlong_as_double(0x7ff8000000000000LL);
-        }
-        else
-        {
-            float G[Q];
-            uint32_t lk;
-            pull_a(f, L, sa, b, i, j, k, G, lk);
-            float rho = 0.f;
-#pragma unroll
-            for (int q = 0; q < Q; ++q) rho += G[q];
-            val = (lk & kSolidSelfBit) ? 0.0 : (double)rho;
-            a.energy[p] += val * val;
-            if (!isfinite(val)) *a.nonfinite = 1;
-        }
-        a.out[row * a.n + p] = val;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0 && a.ctl) a.ctl->step[a.parity ^ 1] = a.ctl->step[a.parity] + 1;
+    const int p = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (p < a.n) probe_warp_a(f, L, sa, b, a, a.direct_row, p, threadIdx.x & 31);
 }
 
 __global__ void __launch_bounds__(128) k_field_rho_a(const float* __restrict__ f, float* __restrict__ out, Layout L,
@@ -760,31 +848,34 @@ __global__ void __launch_bounds__(128) k_field_rho_a(const float* __restrict__ f
 }  // namespace
 
 cudaError_t launch_step_a(const float* fin, float* fout, const Layout& L, const StepArgs& a, const SchemeAArgs& b,
-                          cudaStream_t stream)
+                          const ProbeArgs& pr, cudaStream_t stream)
 {
     if (L.bc != BC) return cudaErrorInvalidValue;
+    if (b.copy && (long long)(L.nx + 2) * (L.ny + 2) >= 1LL << 30) return cudaErrorInvalidValue;   // indexed in 32 bits
     // every instance takes one plane per thread; 04's, with its column values
     // hoisted, at the lean instances' 72 registers (28 warps per SM): on 04's
     // 208^3 grid 0.309 ms (0.293 ms with the paired collision) against 0.326 ms
     // at 96 registers with four planes per thread, 0.320 ms at 80 registers with
     // two, 0.349-0.367 ms otherwise
-    constexpr int kBlock = 128;
+    constexpr int kBlock = kPairBlock;
     const unsigned gx = (unsigned)((L.nx + 2 * kBlock - 1) / (2 * kBlock));
-    if (b.field_mode == 2 || b.sg_xy || b.fld_xy)
-        k_step_a<kBlock, 7, 2, 1><<<dim3(gx, L.ny, L.nz), kBlock, 0, stream>>>(fin, fout, L, a, b);
+    SideBlocks side = side_blocks_a(L, (int)gx, b.copy, pr.n);
+    if (!step_a_has_side(b)) side.rows = 0;
+    const dim3 grid(gx, (unsigned)(L.ny + side.rows), (unsigned)L.nz);
+    if (!step_a_has_side(b))
+        k_step_a<kBlock, 7, 2, 1, false><<<grid, kBlock, 0, stream>>>(fin, fout, L, a, b, pr, side);
     else if (b.blend || b.zper)
-        k_step_a<kBlock, 7, 1, 1><<<dim3(gx, L.ny, L.nz), kBlock, 0, stream>>>(fin, fout, L, a, b);
+        k_step_a<kBlock, 7, 1, 1, true><<<grid, kBlock, 0, stream>>>(fin, fout, L, a, b, pr, side);
     else
-        k_step_a<kBlock, 7, 0, 1><<<dim3(gx, L.ny, L.nz), kBlock, 0, stream>>>(fin, fout, L, a, b);
+        k_step_a<kBlock, 7, 0, 1, true><<<grid, kBlock, 0, stream>>>(fin, fout, L, a, b, pr, side);
     return cudaGetLastError();
 }
 
-cudaError_t launch_copy_a(const float* fin, float* fout, const Layout& L, const StepArgs& a, const SchemeAArgs& b,
-                          cudaStream_t stream)
+cudaError_t launch_side_a(const float* fin, float* fout, const Layout& L, const StepArgs& a, const SchemeAArgs& b,
+                          const ProbeArgs& pr, cudaStream_t stream)
 {
-    const long long n = 2LL * (L.ny + 2) * (L.nz + 2) + 2LL * L.nx * (L.nz + 2) + 2LL * L.nx * L.ny;
-    if (n + 127 > 0x7fffffffLL) return cudaErrorInvalidValue;   // the kernel indexes in 32 bits
-    k_copy_a<<<(unsigned)((n + 127) / 128), 128, 0, stream>>>(fin, fout, L, a, b);
+    const SideBlocks side = side_blocks_a(L, 1, b.copy, pr.n);
+    k_side_a<<<dim3((unsigned)side.rows, (unsigned)L.nz), kPairBlock, 0, stream>>>(fin, fout, L, a, b, pr, side);
     return cudaGetLastError();
 }
 
@@ -799,7 +890,8 @@ cudaError_t launch_init_a(float* f0, float* f1, float* xgh0, float* xgh1, const 
 cudaError_t launch_probe_a(const float* f, const Layout& L, const StepArgs& sa, const SchemeAArgs& b,
                            const ProbeArgs& a, cudaStream_t stream)
 {
-    k_probe_a<<<1, 256, 0, stream>>>(f, L, sa, b, a);
+    if (a.n <= 0) return cudaSuccess;
+    k_probe_a<<<(unsigned)((a.n + 3) / 4), 128, 0, stream>>>(f, L, sa, b, a);
     return cudaGetLastError();
 }
 
