@@ -329,9 +329,11 @@ cudaError_t launch_step_moments(const float* fin, float* fout, const Layout& L, 
                                 PairMoments* mom, cudaStream_t stream);
 cudaError_t launch_probe(int storage, const void* f, const Layout& L, const StepArgs& sa, const ProbeArgs& a,
                          cudaStream_t stream);
-// (float)(rho - 1) of every interior cell, pulled from the pre-step buffer `f`.
+// (float)(rho - 1) of interior rows [row0, row0 + rows), row (k - 1) ny + j - 1, pulled from the pre-step
+// buffer `f`, dense into `out` (device or pinned host memory); kFieldRows rows a launch.
+constexpr int kFieldRows = 65535;
 cudaError_t launch_field_rho(int storage, const void* f, float* out, const Layout& L, const StepArgs& sa,
-                             float scale, cudaStream_t stream);
+                             float scale, int row0, int rows, cudaStream_t stream);
 // Conversions between the stored deviations and FP64 f in the reference's
 // AoS halo-inclusive layout (f[idx*19+q]).
 cudaError_t launch_export_f(int storage, const void* f, double* out, const Layout& L, const XFace& xf, float scale,
@@ -353,7 +355,7 @@ cudaError_t launch_init_a(float* f0, float* f1, float* xgh0, float* xgh1, const 
 cudaError_t launch_probe_a(const float* f, const Layout& L, const StepArgs& sa, const SchemeAArgs& b,
                            const ProbeArgs& a, cudaStream_t stream);
 cudaError_t launch_field_rho_a(const float* f, float* out, const Layout& L, const StepArgs& sa, const SchemeAArgs& b,
-                               cudaStream_t stream);
+                               int row0, int rows, cudaStream_t stream);
 // Periodic z: copy the stored values of the FLUID cells of planes nz and 1
 // into halo planes 0 and nz + 1 (a SOLID cell's slots are its mailbox), for
 // the initial state; the step kernel stores those planes twice itself.

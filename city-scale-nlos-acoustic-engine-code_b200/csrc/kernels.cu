@@ -1229,20 +1229,22 @@ __global__ void __launch_bounds__(128) k_probe(const S* __restrict__ f, Layout L
     if (p < a.n) probe_warp<S>(f, L, sa.links, sa.xf.xgh, a, row, p, threadIdx.x & 31);
 }
 
+// (float)(rho - 1) of rows [row0, row0 + gridDim.y) of the interior, row r =
+// (k - 1) ny + j - 1, dense into `out` (device memory, or pinned host memory).
 template <typename S>
 __global__ void __launch_bounds__(128) k_field_rho(const S* __restrict__ f, float* __restrict__ out, Layout L,
-                                                   StepArgs sa, float inv_scale)
+                                                   StepArgs sa, float inv_scale, int row0)
 {
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
     if (i0 >= L.nx) return;
-    const int j = blockIdx.y + 1, k = blockIdx.z + 1;
+    const int row = row0 + (int)blockIdx.y, k = 1 + row / L.ny, j = 1 + row - (k - 1) * L.ny;
     bool solid;
     float G[Q];
     pull_cell<S>(f, L, sa, i0 + 1, j, k, G, solid);
     float rho = 0.f;
 #pragma unroll
     for (int q = 0; q < Q; ++q) rho += G[q];
-    out[((long long)(k - 1) * L.ny + (j - 1)) * L.nx + i0] = solid ? 0.f : rho * inv_scale;
+    out[(long long)blockIdx.y * L.nx + i0] = solid ? 0.f : rho * inv_scale;
 }
 
 // ---------------------------------------------------------------- import/export
@@ -1501,10 +1503,16 @@ cudaError_t launch_probe(int storage, const void* f, const Layout& L, const Step
 }
 
 cudaError_t launch_field_rho(int storage, const void* f, float* out, const Layout& L, const StepArgs& sa,
-                             float scale, cudaStream_t stream)
+                             float scale, int row0, int rows, cudaStream_t stream)
 {
-    if (storage == 0) k_field_rho<float><<<row_grid(L), 128, 0, stream>>>((const float*)f, out, L, sa, 1.0f / scale);
-    else k_field_rho<__half><<<row_grid(L), 128, 0, stream>>>((const __half*)f, out, L, sa, 1.0f / scale);
+    // the rows of a launch are its blocks along y
+    for (int r = 0; r < rows; r += kFieldRows)
+    {
+        const dim3 g((unsigned)((L.nx + 127) / 128), (unsigned)std::min(kFieldRows, rows - r));
+        float* o = out + (long long)r * L.nx;
+        if (storage == 0) k_field_rho<float><<<g, 128, 0, stream>>>((const float*)f, o, L, sa, 1.0f / scale, row0 + r);
+        else k_field_rho<__half><<<g, 128, 0, stream>>>((const __half*)f, o, L, sa, 1.0f / scale, row0 + r);
+    }
     return cudaGetLastError();
 }
 

@@ -5,6 +5,7 @@
 // (forcing at the collided cell, zero-gradient halos).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "check.cuh"
@@ -831,18 +832,18 @@ __global__ void __launch_bounds__(128) k_probe_a(const float* __restrict__ f, La
 }
 
 __global__ void __launch_bounds__(128) k_field_rho_a(const float* __restrict__ f, float* __restrict__ out, Layout L,
-                                                     StepArgs sa, SchemeAArgs b)
+                                                     StepArgs sa, SchemeAArgs b, int row0)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     if (i > L.nx) return;
-    const int j = blockIdx.y + 1, k = blockIdx.z + 1;
+    const int row = row0 + (int)blockIdx.y, k = 1 + row / L.ny, j = 1 + row - (k - 1) * L.ny;
     float G[Q];
     uint32_t lk;
     pull_a(f, L, sa, b, i, j, k, G, lk);
     float rho = 0.f;
 #pragma unroll
     for (int q = 0; q < Q; ++q) rho += G[q];
-    out[((long long)(k - 1) * L.ny + (j - 1)) * L.nx + (i - 1)] = (lk & kSolidSelfBit) ? 0.f : rho;
+    out[(long long)blockIdx.y * L.nx + (i - 1)] = (lk & kSolidSelfBit) ? 0.f : rho;
 }
 
 }  // namespace
@@ -896,10 +897,13 @@ cudaError_t launch_probe_a(const float* f, const Layout& L, const StepArgs& sa, 
 }
 
 cudaError_t launch_field_rho_a(const float* f, float* out, const Layout& L, const StepArgs& sa, const SchemeAArgs& b,
-                               cudaStream_t stream)
+                               int row0, int rows, cudaStream_t stream)
 {
-    const dim3 g((unsigned)((L.nx + 127) / 128), (unsigned)L.ny, (unsigned)L.nz);
-    k_field_rho_a<<<g, 128, 0, stream>>>(f, out, L, sa, b);
+    for (int r = 0; r < rows; r += kFieldRows)
+    {
+        const dim3 g((unsigned)((L.nx + 127) / 128), (unsigned)std::min(kFieldRows, rows - r));
+        k_field_rho_a<<<g, 128, 0, stream>>>(f, out + (long long)r * L.nx, L, sa, b, row0 + r);
+    }
     return cudaGetLastError();
 }
 
