@@ -238,8 +238,72 @@ __device__ __forceinline__ void adj_ghost_cell(const AdjGhostArgs& a, const Ghos
         a.gadj[off + (long long)p * n + lt] = lh[p] + vk[0] + ex(p) * vk[1] + ey(p) * vk[2] + ez(p) * vk[3];
 }
 
-__global__ void __launch_bounds__(128) k_adj_ghost(AdjGhostArgs a)
+// Residual of probe p enters the adjoint of every population it summed.
+__device__ __forceinline__ void add_residual(const AdjProbeArgs& a, int p)
 {
+    if (p >= a.n) return;
+    const int i = a.ijk[3 * p], j = a.ijk[3 * p + 1], k = a.ijk[3 * p + 2];
+    const float r = (float)a.resid[p];
+    if (i < 0 || r == 0.f) return;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) atomicAdd(&a.lam[a.L.elem(q, i, j, k)], r);
+}
+
+// Source gradient of one step: Lam_c = sum_q w_q lamH^s[q](c) over the
+// injection cells; out = (sum_c w_hat_c Lam_c, sum_c dw_hat_c/dpos Lam_c),
+// reduced in FP64, by one block of 128 threads.
+__device__ __forceinline__ void source_gradient(const AdjSourceArgs& a)
+{
+    __shared__ double red[4][4];
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    const AdjSourceCell* cells = a.cells + (long long)a.step * a.ncell;
+    for (int c = threadIdx.x; c < a.ncell; c += blockDim.x)
+    {
+        const AdjSourceCell e = cells[c];
+        if (e.i < 0) continue;
+        float lg[Q];
+        gather_lam(a.L, a.links, a.lam_in, a.gadj, a.gadj_off, e.i, e.j, e.k, lg);
+        double lam = 0.0;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) lam += wd(q) * (double)lg[q];
+        acc[0] += e.what * lam;
+        acc[1] += e.dwhat[0] * lam;
+        acc[2] += e.dwhat[1] * lam;
+        acc[3] += e.dwhat[2] * lam;
+    }
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+        for (int o = 16; o > 0; o >>= 1) acc[m] += __shfl_xor_sync(kFull, acc[m], o);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0)
+#pragma unroll
+        for (int m = 0; m < 4; ++m) red[warp][m] = acc[m];
+    __syncthreads();
+    if (threadIdx.x < 4)
+    {
+        double t = 0.0;
+        for (int w = 0; w < 4; ++w) t += red[w][threadIdx.x];
+        a.out[4LL * a.step + threadIdx.x] = t;
+    }
+}
+
+// What comes between two adjoint steps, one launch: the ghost adjoints of step
+// s, the probe residuals of step s and the source terms of the step before
+// (s + 1), each where it touches nothing that another of them writes (the
+// caller's AdjBetweenArgs); blocks [0, nghost) the ghosts, then the residuals,
+// then one for the source.  As launches of their own the last two took a
+// second stream and two event pairs a step.
+__global__ void __launch_bounds__(128, 8) k_adj_between(const __grid_constant__ AdjGhostArgs a,
+                                                     const __grid_constant__ AdjProbeArgs pa,
+                                                     const __grid_constant__ AdjSourceArgs sa, int nghost, int nprobe)
+{
+    if ((int)blockIdx.x >= nghost)
+    {
+        const int b = (int)blockIdx.x - nghost;
+        if (b < nprobe) add_residual(pa, b * 128 + (int)threadIdx.x);
+        else source_gradient(sa);
+        return;
+    }
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= a.ga.total) return;
     int fi = 0;
@@ -560,62 +624,17 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_adj_step(AdjStepArgs a)
     }
 }
 
-// Residual of each probe enters the adjoint of every population it summed.
-__global__ void k_adj_probe(float* __restrict__ lam, AdjProbeArgs a)
-{
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= a.n) return;
-    const int i = a.ijk[3 * p], j = a.ijk[3 * p + 1], k = a.ijk[3 * p + 2];
-    const float r = (float)a.resid[p];
-    if (i < 0 || r == 0.f) return;
-#pragma unroll
-    for (int q = 0; q < Q; ++q) atomicAdd(&lam[a.L.elem(q, i, j, k)], r);
-}
-
-// Source gradient of one step: Lam_c = sum_q w_q lamH^s[q](c) over the
-// injection cells; out = (sum_c w_hat_c Lam_c, sum_c dw_hat_c/dpos Lam_c),
-// reduced in FP64.
-__global__ void __launch_bounds__(128) k_adj_source(AdjSourceArgs a)
-{
-    __shared__ double red[4][4];
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    const AdjSourceCell* cells = a.cells + (long long)a.step * a.ncell;
-    for (int c = threadIdx.x; c < a.ncell; c += blockDim.x)
-    {
-        const AdjSourceCell e = cells[c];
-        if (e.i < 0) continue;
-        float lg[Q];
-        gather_lam(a.L, a.links, a.lam_in, a.gadj, a.gadj_off, e.i, e.j, e.k, lg);
-        double lam = 0.0;
-#pragma unroll
-        for (int q = 0; q < Q; ++q) lam += wd(q) * (double)lg[q];
-        acc[0] += e.what * lam;
-        acc[1] += e.dwhat[0] * lam;
-        acc[2] += e.dwhat[1] * lam;
-        acc[3] += e.dwhat[2] * lam;
-    }
-#pragma unroll
-    for (int m = 0; m < 4; ++m)
-        for (int o = 16; o > 0; o >>= 1) acc[m] += __shfl_xor_sync(kFull, acc[m], o);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0)
-#pragma unroll
-        for (int m = 0; m < 4; ++m) red[warp][m] = acc[m];
-    __syncthreads();
-    if (threadIdx.x < 4)
-    {
-        double t = 0.0;
-        for (int w = 0; w < 4; ++w) t += red[w][threadIdx.x];
-        a.out[4LL * a.step + threadIdx.x] = t;
-    }
-}
-
 }  // namespace
 
-cudaError_t launch_adj_ghost(const AdjGhostArgs& a, cudaStream_t stream)
+cudaError_t launch_adj_between(const AdjGhostArgs* ghost, const AdjProbeArgs* resid, const AdjSourceArgs* source,
+                               cudaStream_t stream)
 {
-    if (a.ga.total <= 0) return cudaSuccess;
-    k_adj_ghost<<<(unsigned)((a.ga.total + 127) / 128), 128, 0, stream>>>(a);
+    const int nghost = ghost ? (int)((ghost->ga.total + 127) / 128) : 0;
+    const int nprobe = resid ? (resid->n + 127) / 128 : 0;
+    const int blocks = nghost + nprobe + (source ? 1 : 0);
+    if (blocks == 0) return cudaSuccess;
+    k_adj_between<<<blocks, 128, 0, stream>>>(ghost ? *ghost : AdjGhostArgs{}, resid ? *resid : AdjProbeArgs{},
+                                              source ? *source : AdjSourceArgs{}, nghost, nprobe);
     return cudaGetLastError();
 }
 
@@ -628,19 +647,6 @@ cudaError_t launch_adj_step(const AdjStepArgs& a, cudaStream_t stream)
     const dim3 g((unsigned)((a.L.nx + 2 * block - 1) / (2 * block)), (unsigned)a.L.ny, (unsigned)a.L.nz);
     if (block == 64) k_adj_step<64, 10><<<g, 64, 0, stream>>>(a);
     else k_adj_step<128, 6><<<g, 128, 0, stream>>>(a);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_adj_source(const AdjSourceArgs& a, cudaStream_t stream)
-{
-    k_adj_source<<<1, 128, 0, stream>>>(a);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_adj_probe(float* lam, const AdjProbeArgs& a, cudaStream_t stream)
-{
-    if (a.n <= 0) return cudaSuccess;
-    k_adj_probe<<<(a.n + 127) / 128, 128, 0, stream>>>(lam, a);
     return cudaGetLastError();
 }
 

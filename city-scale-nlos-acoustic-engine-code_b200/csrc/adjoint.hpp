@@ -74,14 +74,18 @@ struct AdjProbeArgs
     const int* ijk;         // [n][3], i = -1: not owned
     const double* resid;    // [n] residuals of this step (0 for SOLID or unowned probes)
     Layout L;
+    float* lam;             // lamF of this step
 };
 
-cudaError_t launch_adj_ghost(const AdjGhostArgs& a, cudaStream_t stream);
+// One launch of what a step's adjoint needs before its J_C^T: the ghost adjoints and the probe residuals of
+// step s and the source terms of step s + 1, null: not in this launch.  Residuals may go with the ghosts where
+// no probe's cell lies in an open face's first interior layer, the source terms (of a step whose buffers the
+// next J_C^T overwrites) where no injection cell does.
+cudaError_t launch_adj_between(const AdjGhostArgs* ghost, const AdjProbeArgs* resid, const AdjSourceArgs* source,
+                               cudaStream_t stream);
 // J_C^T of the gathered lamF^s (plus, at the open faces, the ghost-adjoint
 // terms written by launch_adj_ghost for the same step) over every interior
 // cell.
 cudaError_t launch_adj_step(const AdjStepArgs& a, cudaStream_t stream);
-cudaError_t launch_adj_source(const AdjSourceArgs& a, cudaStream_t stream);
-cudaError_t launch_adj_probe(float* lam, const AdjProbeArgs& a, cudaStream_t stream);
 
 }  // namespace lbm

@@ -1232,10 +1232,10 @@ cudaError_t timed_step_launch(lbm_handle* h, int parity, bool batched, long long
     const auto launch = [&]() {
         if (!h->scheme_a() && batched)
             return launch_batched_step(h->storage, h->f[parity], h->f[parity ^ 1], h->L, h->step_args(parity), h->scale,
-                                       fused_args(h, parity), fused_steps(h), h->stream);
+                                       fused_args(h, parity), fused_steps(h), nullptr, h->stream);
         if (!h->scheme_a())
             return launch_step(h->storage, h->f[parity], h->f[parity ^ 1], h->L, h->step_args(parity), h->scale,
-                               h->stream);
+                               nullptr, h->stream);
         StepArgs sa;
         SchemeAArgs b;
         scheme_a_args(h, parity, batched, s, sa, b);
@@ -2335,6 +2335,7 @@ AdjPlan adjoint_plan(const lbm_handle* h, int T, int ckpt_outer, int ckpt_inner)
         c.get<double>((size_t)T * np);
         c.get<AdjSourceCell>((size_t)T * p.ncell);
         c.get<double>((size_t)T * 4);
+        c.get<SourceEntry>((size_t)T);
         return c.used;
     };
     p.Tt = T;
@@ -2474,6 +2475,7 @@ extern "C" int lbm_adjoint_grad(lbm_handle* h, int nsteps, const double* observe
     float* gadj;
     double *d_pred, *d_resid, *d_out;
     AdjSourceCell* d_cells;
+    SourceEntry* d_entries;
     const auto carve = [&](Carve& c) {
         outer = StateSlots{c.get<float>((size_t)Mr * plan.ck_slot), pop, plan.ck_slot - pop};
         inner = StateSlots{c.get<float>((size_t)(Mr > 0 ? NI : 0) * plan.ck_slot), pop, plan.ck_slot - pop};
@@ -2485,6 +2487,7 @@ extern "C" int lbm_adjoint_grad(lbm_handle* h, int nsteps, const double* observe
         d_resid = c.get<double>((size_t)T * np);
         d_cells = c.get<AdjSourceCell>(cells.size());
         d_out = c.get<double>((size_t)T * 4);
+        d_entries = c.get<SourceEntry>((size_t)T);
     };
     {
         Carve count;
@@ -2528,10 +2531,19 @@ extern "C" int lbm_adjoint_grad(lbm_handle* h, int nsteps, const double* observe
                                 h->stream);
         return r;
     };
-    // The ghost fill reads only the first interior layer of each open face (the
-    // x faces through their export arrays, which the source also updates);
-    // when step s's injection cells stay off that layer, source and ghost fill
-    // touch disjoint cells and the source runs on the side stream beside it.
+    // The ghost fill and its adjoint touch only the first interior layer of each
+    // open face (the x faces through their export arrays, which the source also
+    // updates); injection cells and probes off that layer can be worked on beside them.
+    const auto on_face = [&](int i, int j, int k) {
+        for (int f = 0; f < h->ga.nfaces; ++f)
+        {
+            const GhostFace& F = h->ga.face[f];
+            const int v = F.axis == 0 ? i : F.axis == 1 ? j : k;
+            const int n = F.axis == 0 ? L.nx : F.axis == 1 ? L.ny : L.nz;
+            if (v == (F.side ? n : 1)) return true;
+        }
+        return false;
+    };
     std::vector<char> source_apart((size_t)T, 0);
     for (int s = 0; s < T; ++s)
     {
@@ -2539,84 +2551,64 @@ extern "C" int lbm_adjoint_grad(lbm_handle* h, int nsteps, const double* observe
         for (int b = 0; b < ncell && apart; ++b)
         {
             const AdjSourceCell& cc = cells[(size_t)s * ncell + b];
-            if (cc.i < 0) continue;
-            for (int f = 0; f < h->ga.nfaces; ++f)
-            {
-                const GhostFace& F = h->ga.face[f];
-                const int v = F.axis == 0 ? cc.i : F.axis == 1 ? cc.j : cc.k;
-                const int n = F.axis == 0 ? L.nx : F.axis == 1 ? L.ny : L.nz;
-                if (v == (F.side ? n : 1)) apart = false;
-            }
+            if (cc.i >= 0 && on_face(cc.i, cc.j, cc.k)) apart = false;
         }
         source_apart[(size_t)s] = apart;
     }
-    // source + ghost fill of step s on the current buffer (G^s -> Ht^s)
-    const auto source_then_ghost = [&](int s, const GhostArgs& g) {
+    bool probes_apart = true;
+    for (int p = 0; p < np; ++p)
+        if (h->probe_owned[p] && on_face(h->probe_ijk[3 * p], h->probe_ijk[3 * p + 1], h->probe_ijk[3 * p + 2]))
+            probes_apart = false;
+    // source + ghost fill of step s on the current buffer (G^s -> Ht^s); the source runs on the side
+    // stream beside the ghost fill where they touch disjoint cells
+    const auto source_then_ghost = [&](int s, float4* face_mom) {
         sargs.direct[0] = entries[s];
+        GhostArgs g = h->ga;
+        g.face_mom = face_mom;
+        g.xf = h->xface(h->cur);
+        const StepArgs sa = h->step_args(h->cur);
         cudaError_t r = cudaSuccess;
         const bool beside = h->ga.total > 0 && source_apart[(size_t)s];
         if (beside)
         {
             r = cudaEventRecord(h->ev_fork, h->stream);
             if (r == cudaSuccess) r = cudaStreamWaitEvent(h->side, h->ev_fork, 0);
-            if (r == cudaSuccess) r = launch_source(h->storage, h->f[h->cur], L, h->step_args(h->cur), sargs, 0, nullptr, h->side);
+            if (r == cudaSuccess) r = launch_source(h->storage, h->f[h->cur], L, sa, sargs, 0, nullptr, h->side);
             if (r == cudaSuccess) r = cudaEventRecord(h->ev_join, h->side);
         }
         else
         {
-            r = launch_source(h->storage, h->f[h->cur], L, h->step_args(h->cur), sargs, 0, nullptr, h->stream);
+            r = launch_source(h->storage, h->f[h->cur], L, sa, sargs, 0, nullptr, h->stream);
         }
         kernels++;
         if (r == cudaSuccess && h->ga.total > 0)
         {
-            GhostArgs gp = g;
-            gp.xf = h->xface(h->cur);
-            r = launch_ghost(h->storage, h->f[h->cur], L, gp, h->stream);
+            r = launch_ghost(h->storage, h->f[h->cur], L, g, h->stream);
             kernels++;
         }
         if (r == cudaSuccess && beside) r = cudaStreamWaitEvent(h->stream, h->ev_join, 0);
         return r;
     };
-    const auto source_ghost = [&](int s) { return source_then_ghost(s, h->ga); };
-    // pull + collide of step s (Ht^s -> G^{s+1}), optionally with its probe record
-    // The probe record of step s reads the step's input buffer, which the step
-    // only reads: it runs on the side stream beside the step, joined before
-    // anything can overwrite that buffer (the next step writes into it).
-    const auto probe_beside = [&](int s) {
-        ProbeArgs pa = probe_args(h, false, s);
-        pa.out = d_pred;
-        cudaError_t r = cudaEventRecord(h->ev_fork, h->stream);
-        if (r == cudaSuccess) r = cudaStreamWaitEvent(h->side, h->ev_fork, 0);
-        if (r == cudaSuccess) r = launch_probe(h->storage, h->f[h->cur], L, h->step_args(h->cur), pa, h->side);
-        if (r == cudaSuccess) r = cudaEventRecord(h->ev_join, h->side);
-        kernels++;
-        return r;
-    };
-    const auto collide = [&](int s, bool probe) {
-        cudaError_t r = probe ? probe_beside(s) : cudaSuccess;
-        if (r == cudaSuccess)
-            r = launch_step(h->storage, h->f[h->cur], h->f[h->cur ^ 1], L, h->step_args(h->cur), h->scale, h->stream);
-        kernels++;
-        if (r == cudaSuccess && probe) r = cudaStreamWaitEvent(h->stream, h->ev_join, 0);
-        h->cur ^= 1;
-        return r;
-    };
-    // Recompute of step s for the reverse pass: source and ghost fill
-    // recording the moments of H^s at the ghosts' interior cells, then the
-    // fused step recording the moments of F^s, both into store slot `slot`.
-    const auto stored_source_ghost = [&](int s, long long slot) {
-        GhostArgs g = h->ga;
-        g.face_mom = face_mom_of(slot);
-        return source_then_ghost(s, g);
-    };
-    // probe_step >= 0: also the probe record of that step (first pass)
-    const auto stored_collide = [&](long long slot, int probe_step = -1) {
-        kernels++;
-        cudaError_t r = probe_step >= 0 ? probe_beside(probe_step) : cudaSuccess;
-        if (r == cudaSuccess)
-            r = launch_step_moments((const float*)h->f[h->cur], (float*)h->f[h->cur ^ 1], L, h->step_args(h->cur), mom_of(slot),
+    const auto source_ghost = [&](int s) { return source_then_ghost(s, nullptr); };
+    // pull + collide of step s (Ht^s -> G^{s+1}), with the moments of F^s into `mom` (null: not kept) and, in
+    // the first pass, its probe record
+    const auto collide = [&](int s, bool probe, PairMoments* mom) {
+        const int p = h->cur;
+        cudaError_t r;
+        if (probe)
+        {
+            FusedArgs fa{};
+            fa.direct_step = s;
+            fa.probe = probe_args(h, false, s);
+            fa.probe.out = d_pred;
+            r = launch_batched_step(h->storage, h->f[p], h->f[p ^ 1], L, h->step_args(p), h->scale, fa, false, mom,
                                     h->stream);
-        if (r == cudaSuccess && probe_step >= 0) r = cudaStreamWaitEvent(h->stream, h->ev_join, 0);
+        }
+        else
+        {
+            r = launch_step(h->storage, h->f[p], h->f[p ^ 1], L, h->step_args(p), h->scale, mom, h->stream);
+        }
+        kernels++;
         h->cur ^= 1;
         return r;
     };
@@ -2625,6 +2617,46 @@ extern "C" int lbm_adjoint_grad(lbm_handle* h, int nsteps, const double* observe
 
     // ---- forward pass: probe predictions, outer checkpoints G^{max(mK1-1,0)}
     // of the segments before the tail, and the tail's forward data
+    if (Mr == 0 && fused_steps(h))
+    {
+        // every step's forward data is kept and no state is checkpointed between
+        // steps: one launch a step, as in a batch of lbm_step
+        NvtxRange phase("adjoint forward pass");
+        CK(cudaMemcpyAsync(d_entries, entries.data(), entries.size() * sizeof(SourceEntry), cudaMemcpyHostToDevice,
+                           h->stream),
+           "adjoint upload");
+        h->ctl_host->step[0] = h->ctl_host->step[1] = 0;
+        h->ctl_host->last = T - 1;
+        h->ctl_host->table_base = h->ctl_host->probe_base = 0;
+        CK(cudaMemcpyAsync(h->ctl, h->ctl_host, offsetof(Control, nonfinite), cudaMemcpyHostToDevice, h->stream),
+           "control");
+        SourceArgs schedule = source_args(h, true);
+        schedule.table = d_entries;
+        CK(launch_source(h->storage, h->f[h->cur], L, h->step_args(h->cur), schedule, h->cur, h->d_next + h->cur,
+                         h->stream),
+           "adjoint forward");
+        GhostArgs g = h->ga;
+        g.face_mom = face_mom_of(0);
+        g.xf = h->xface(h->cur);
+        CK(launch_ghost(h->storage, h->f[h->cur], L, g, h->stream), "adjoint forward");
+        kernels += 2;
+        for (int s = 0; s < T; ++s)
+        {
+            const int p = h->cur;
+            FusedArgs fa = fused_args(h, p);
+            fa.src = schedule;
+            fa.probe.out = d_pred;
+            fa.face_mom = s + 1 < T ? face_mom_of(s + 1) : nullptr;
+            for (int f = 0; f < h->ga.nfaces; ++f)
+                fa.face_first[h->ga.face[f].axis * 2 + h->ga.face[f].side] = h->ga.face[f].first;
+            CK(launch_batched_step(h->storage, h->f[p], h->f[p ^ 1], L, h->step_args(p), h->scale, fa, true, mom_of(s),
+                                   h->stream),
+               "adjoint forward");
+            kernels++;
+            h->cur ^= 1;
+        }
+    }
+    else
     {
         NvtxRange phase("adjoint forward pass");
         int m = 0;
@@ -2635,16 +2667,9 @@ extern "C" int lbm_adjoint_grad(lbm_handle* h, int nsteps, const double* observe
                 CK(save_g(outer, m), "checkpoint");
                 ++m;
             }
-            if (Tt < T && s >= cnT)
-            {
-                CK(stored_source_ghost(s, s - cnT), "adjoint forward");
-                CK(stored_collide(s - cnT, s), "adjoint forward");
-            }
-            else
-            {
-                CK(source_ghost(s), "adjoint forward");
-                CK(collide(s, true), "adjoint forward");
-            }
+            const bool stored = Tt < T && s >= cnT;
+            CK(source_then_ghost(s, stored ? face_mom_of(s - cnT) : nullptr), "adjoint forward");
+            CK(collide(s, true, stored ? mom_of(s - cnT) : nullptr), "adjoint forward");
         }
     }
 
@@ -2671,31 +2696,34 @@ extern "C" int lbm_adjoint_grad(lbm_handle* h, int nsteps, const double* observe
     NvtxRange reverse_phase("adjoint reverse pass");
     for (int b = 0; b < 2; ++b) CK(cudaMemsetAsync(lam[b], 0, pop * sizeof(float), h->stream), "adjoint memset");
     int la = 0;
-    AdjProbeArgs pa{np, h->d_probe_ijk, nullptr, L};
-    pa.resid = d_resid + (size_t)(T - 1) * np;
-    CK(launch_adj_probe(lam[la], pa, h->stream), "adjoint probe");
-    kernels++;
+    AdjSourceArgs late{};        // source terms of the step before, still to be computed
+    bool late_due = false;
     // adjoint steps a1-1 .. a0 with the forward data of step s in store slot s - cn
     const auto reverse_segment = [&](int a0, int a1, int cn) -> int {
         for (int s = a1 - 1; s >= a0; --s)
         {
-            if (h->ga.total > 0)
+            AdjGhostArgs ga{L, h->ga, h->links, lam[la], face_mom_of(s - cn), gadj, {}};
+            std::copy(gadj_off, gadj_off + 6, ga.gadj_off);
+            const AdjGhostArgs* ghosts = h->ga.total > 0 ? &ga : nullptr;
+            const AdjProbeArgs pa{np, h->d_probe_ijk, d_resid + (size_t)s * np, L, lam[la]};
+            if (ghosts && !probes_apart)
             {
-                AdjGhostArgs ga{L, h->ga, h->links, lam[la], face_mom_of(s - cn), gadj, {}};
-                std::copy(gadj_off, gadj_off + 6, ga.gadj_off);
-                CK(launch_adj_ghost(ga, h->stream), "adjoint ghost");
+                CK(launch_adj_between(nullptr, &pa, nullptr, h->stream), "adjoint probe");
                 kernels++;
             }
-            // the source terms read lamF^s and the ghost-adjoint terms, which the
-            // adjoint step and the probe residuals do not write: they run on the
-            // side stream beside them, joined before the next ghost pass
-            AdjSourceArgs sa{L, h->links, lam[la], gadj, {}, d_cells, ncell, s, d_out};
-            std::copy(gadj_off, gadj_off + 6, sa.gadj_off);
-            CK(cudaEventRecord(h->ev_fork, h->stream), "adjoint fork");
-            CK(cudaStreamWaitEvent(h->side, h->ev_fork, 0), "adjoint fork");
-            CK(launch_adj_source(sa, h->side), "adjoint source");
-            CK(cudaEventRecord(h->ev_join, h->side), "adjoint join");
+            CK(launch_adj_between(ghosts, ghosts && !probes_apart ? nullptr : &pa, late_due ? &late : nullptr, h->stream),
+               "adjoint ghost");
             kernels++;
+            // the source terms read lamF^s, which the adjoint step of s only reads, and at the open faces the
+            // ghost adjoints of s, which the next launch of them overwrites
+            late = AdjSourceArgs{L, h->links, lam[la], gadj, {}, d_cells, ncell, s, d_out};
+            std::copy(gadj_off, gadj_off + 6, late.gadj_off);
+            late_due = source_apart[(size_t)s] != 0;
+            if (!late_due)
+            {
+                CK(launch_adj_between(nullptr, nullptr, &late, h->stream), "adjoint source");
+                kernels++;
+            }
             if (s > 0)
             {
                 AdjStepArgs as{L, h->sa, lam[la], lam[la ^ 1], mom_of(s - 1 - cn), gadj, {}, adj_prefetch};
@@ -2703,11 +2731,7 @@ extern "C" int lbm_adjoint_grad(lbm_handle* h, int nsteps, const double* observe
                 CK(launch_adj_step(as, h->stream), "adjoint step");
                 kernels++;
                 la ^= 1;
-                pa.resid = d_resid + (size_t)(s - 1) * np;
-                CK(launch_adj_probe(lam[la], pa, h->stream), "adjoint probe");
-                kernels++;
             }
-            CK(cudaStreamWaitEvent(h->stream, h->ev_join, 0), "adjoint join");
         }
         return LBM_OK;
     };
@@ -2728,7 +2752,7 @@ extern "C" int lbm_adjoint_grad(lbm_handle* h, int nsteps, const double* observe
             for (; at < cn; ++at)
             {
                 CK(source_ghost((int)at), "recompute");
-                CK(collide((int)at, false), "recompute");
+                CK(collide((int)at, false, nullptr), "recompute");
             }
             CK(save_g(inner, n), "checkpoint");
         }
@@ -2739,12 +2763,18 @@ extern "C" int lbm_adjoint_grad(lbm_handle* h, int nsteps, const double* observe
             CK(restore_g(inner, n), "restore");
             for (int s = cn; s < a1; ++s)
             {
-                CK(stored_source_ghost(s, s - cn), "recompute");
-                if (s + 1 < a1) CK(stored_collide(s - cn), "recompute");
+                CK(source_then_ghost(s, face_mom_of(s - cn)), "recompute");
+                if (s + 1 < a1) CK(collide(s, false, mom_of(s - cn)), "recompute");
             }
             st = reverse_segment(a0, a1, cn);
             if (st) return st;
         }
+    }
+
+    if (late_due)
+    {
+        CK(launch_adj_between(nullptr, nullptr, &late, h->stream), "adjoint source");
+        kernels++;
     }
 
     // ---- gradients: d L / d val_s = mu_s dt gain; d L / d pos = sum_s mass_s nu_s

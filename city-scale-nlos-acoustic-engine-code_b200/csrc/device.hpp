@@ -298,19 +298,7 @@ cudaError_t launch_build_links(const uint8_t* mask_ref, uint32_t* links, uint32_
 cudaError_t launch_source(int storage, void* f, const Layout& L, const StepArgs& sa, const SourceArgs& a,
                           int parity, SourceNext* next, cudaStream_t stream);
 cudaError_t launch_ghost(int storage, void* f, const Layout& L, const GhostArgs& a, cudaStream_t stream);
-// Fused step: FP32 storage runs the two-cells-per-thread pair kernel, FP16
-// storage the warp pipelines of cp.async copies.
-cudaError_t launch_step(int storage, const void* fin, void* fout, const Layout& L, const StepArgs& a,
-                        float scale, cudaStream_t stream);
-// A batched step: the same with the probes recorded and the step counter advanced; fused: also with the next
-// step's sources and ghosts applied to its results.
-cudaError_t launch_batched_step(int storage, const void* fin, void* fout, const Layout& L, const StepArgs& a,
-                                float scale, const FusedArgs& fa, bool fused, cudaStream_t stream);
-// One-time set-up of the fused step on the current device (shared-memory
-// attribute, occupancy); call before the first launch or capture.
-cudaError_t prepare_step(int storage);
-// Fused step (FP32 storage, the default implementation) that also writes the
-// moments (rho', jx, jy, jz) of every cell's pulled populations to `mom`: the
+// Moments (rho', jx, jy, jz) of every cell's pulled populations: the
 // forward data of the adjoint's BGK Jacobian, where they enter only through
 // terms of the wave's amplitude (J^2, J / r, 1 / r with r = 1 + rho').  Each
 // value is kept as a 12-bit float (sign, FP16's 5-bit exponent, 6 mantissa
@@ -325,8 +313,18 @@ struct PairMoments
 {
     unsigned w[3];
 };
-cudaError_t launch_step_moments(const float* fin, float* fout, const Layout& L, const StepArgs& a,
-                                PairMoments* mom, cudaStream_t stream);
+// Fused step: FP32 storage runs the two-cells-per-thread pair kernel, FP16
+// storage the warp pipelines of cp.async copies.  mom (FP32 storage, else
+// null): also receives the moments.
+cudaError_t launch_step(int storage, const void* fin, void* fout, const Layout& L, const StepArgs& a,
+                        float scale, PairMoments* mom, cudaStream_t stream);
+// A batched step: the same with the probes recorded and the step counter advanced; fused: also with the next
+// step's sources and ghosts applied to its results.
+cudaError_t launch_batched_step(int storage, const void* fin, void* fout, const Layout& L, const StepArgs& a,
+                                float scale, const FusedArgs& fa, bool fused, PairMoments* mom, cudaStream_t stream);
+// One-time set-up of the fused step on the current device (shared-memory
+// attribute, occupancy); call before the first launch or capture.
+cudaError_t prepare_step(int storage);
 cudaError_t launch_probe(int storage, const void* f, const Layout& L, const StepArgs& sa, const ProbeArgs& a,
                          cudaStream_t stream);
 // (float)(rho - 1) of interior rows [row0, row0 + rows), row (k - 1) ny + j - 1, pulled from the pre-step

@@ -1448,30 +1448,26 @@ cudaError_t prepare_step(int storage)
 namespace {
 template <int MODE>
 cudaError_t launch_step_mode(int storage, const void* fin, void* fout, const Layout& L, const StepArgs& a, float scale,
-                             const FusedArgs& fa, cudaStream_t stream)
+                             const FusedArgs& fa, PairMoments* mom, cudaStream_t stream)
 {
+    if (storage == 0 && mom) return launch_pair_step<true, MODE>((const float*)fin, (float*)fout, L, a, mom, fa, stream);
     if (storage == 0) return launch_pair_step<false, MODE>((const float*)fin, (float*)fout, L, a, nullptr, fa, stream);
+    if (mom) return cudaErrorInvalidValue;
     return launch_hw<2, 4, 5, MODE>((const __half*)fin, (__half*)fout, L, a, 1.0f / scale, fa, stream);
 }
 }  // namespace
 
 cudaError_t launch_step(int storage, const void* fin, void* fout, const Layout& L, const StepArgs& a,
-                        float scale, cudaStream_t stream)
+                        float scale, PairMoments* mom, cudaStream_t stream)
 {
-    return launch_step_mode<kPlain>(storage, fin, fout, L, a, scale, FusedArgs{}, stream);
+    return launch_step_mode<kPlain>(storage, fin, fout, L, a, scale, FusedArgs{}, mom, stream);
 }
 
 cudaError_t launch_batched_step(int storage, const void* fin, void* fout, const Layout& L, const StepArgs& a,
-                                float scale, const FusedArgs& fa, bool fused, cudaStream_t stream)
+                                float scale, const FusedArgs& fa, bool fused, PairMoments* mom, cudaStream_t stream)
 {
-    if (fused) return launch_step_mode<kFused>(storage, fin, fout, L, a, scale, fa, stream);
-    return launch_step_mode<kSide>(storage, fin, fout, L, a, scale, fa, stream);
-}
-
-cudaError_t launch_step_moments(const float* fin, float* fout, const Layout& L, const StepArgs& a,
-                                PairMoments* mom, cudaStream_t stream)
-{
-    return launch_pair_step<true, kPlain>(fin, fout, L, a, mom, FusedArgs{}, stream);
+    if (fused) return launch_step_mode<kFused>(storage, fin, fout, L, a, scale, fa, mom, stream);
+    return launch_step_mode<kSide>(storage, fin, fout, L, a, scale, fa, mom, stream);
 }
 
 cudaError_t launch_source(int storage, void* f, const Layout& L, const StepArgs& sa, const SourceArgs& a,
