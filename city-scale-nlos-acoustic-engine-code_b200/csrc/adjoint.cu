@@ -641,12 +641,16 @@ cudaError_t launch_adj_between(const AdjGhostArgs* ghost, const AdjProbeArgs* re
 cudaError_t launch_adj_step(const AdjStepArgs& a, cudaStream_t stream)
 {
     // 80 registers, no spills, 24 warps per SM (a 3000-step gradient on the
-    // 256x256x128 patch: 1578 ms against 1587 ms at 96 registers); rows of up
-    // to 128 columns take 64-thread blocks, so no warp idles
-    const int block = a.L.nx <= 128 ? 64 : 128;
-    const dim3 g((unsigned)((a.L.nx + 2 * block - 1) / (2 * block)), (unsigned)a.L.ny, (unsigned)a.L.nz);
-    if (block == 64) k_adj_step<64, 10><<<g, 64, 0, stream>>>(a);
-    else k_adj_step<128, 6><<<g, 128, 0, stream>>>(a);
+    // 256x256x128 patch: 1578 ms against 1587 ms at 96 registers)
+    const int warps = row_block_warps(a.L.nx), cells = 64 * warps;
+    const dim3 g((unsigned)((a.L.nx + cells - 1) / cells), (unsigned)a.L.ny, (unsigned)a.L.nz);
+    switch (warps)
+    {
+    case 2: k_adj_step<64, 10><<<g, 64, 0, stream>>>(a); break;
+    case 3: k_adj_step<96, 8><<<g, 96, 0, stream>>>(a); break;
+    case 5: k_adj_step<160, 5><<<g, 160, 0, stream>>>(a); break;
+    default: k_adj_step<128, 6><<<g, 128, 0, stream>>>(a); break;
+    }
     return cudaGetLastError();
 }
 

@@ -289,6 +289,21 @@ __device__ __forceinline__ int pair_row()
 }
 #endif
 
+// Warps per block of the scheme-A and adjoint steps, whose blocks lie along a
+// row (64 columns a warp): of 2 to 5 the one that leaves the fewest warps of a
+// row without cells, 4 where it is among them.  Blocks of four against that
+// choice: Doppler 80x80x120 42.5 / 32.3 us a step, 180x180x270 257 / 238,
+// 04's program on 83^3 42.2 / 34.7, 125^3 84.5 / 72.9, 166^3 163 / 151, 01's on
+// 320x320x8 (five segments) 32.8 / 31.1, a 300x200x64 gradient step 268 / 260.
+inline int row_block_warps(int nx)
+{
+    const int seg = (nx + 63) / 64;
+    int best = 4;
+    for (const int w : {5, 3, 2})
+        if ((seg + w - 1) / w * w < (seg + best - 1) / best * best) best = w;
+    return best;
+}
+
 // ---- launchers (kernels.cu) ----------------------------------------------
 // storage: 0 = float, 1 = __half.  All launches go to `stream`.
 cudaError_t launch_build_links(const uint8_t* mask_ref, uint32_t* links, uint32_t* near, const Layout& L,

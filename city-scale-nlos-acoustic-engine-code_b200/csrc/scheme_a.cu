@@ -7,6 +7,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "check.cuh"
 #include "device.hpp"
@@ -589,11 +590,11 @@ struct SideBlocks
     int copy, probe;   // blocks of either kind per layer
     HaloLayer halo;
 };
-SideBlocks side_blocks_a(const Layout& L, int gx, int copy, int nprobe)
+SideBlocks side_blocks_a(const Layout& L, int gx, int warps, int copy, int nprobe)
 {
     const HaloLayer h = halo_layer(L);
-    const int nc = copy ? (h.ring + h.share + kPairBlock - 1) / kPairBlock : 0;
-    const int np = (1 + (nprobe + 3) / 4 + L.nz - 1) / L.nz;
+    const int nc = copy ? (h.ring + h.share + 32 * warps - 1) / (32 * warps) : 0;
+    const int np = (1 + (nprobe + warps - 1) / warps + L.nz - 1) / L.nz;
     return SideBlocks{(nc + np + gx - 1) / gx, nc, np, h};
 }
 __device__ __forceinline__ void side_block_a(const float* __restrict__ fin, float* __restrict__ fout, const Layout& L,
@@ -602,7 +603,7 @@ __device__ __forceinline__ void side_block_a(const float* __restrict__ fin, floa
 {
     if (block < n.copy)
     {
-        copy_halo_cell(fin, fout, L, a, b, n.halo, layer, block * kPairBlock + (int)threadIdx.x);
+        copy_halo_cell(fin, fout, L, a, b, n.halo, layer, block * (int)blockDim.x + (int)threadIdx.x);
         return;
     }
     if (block >= n.copy + n.probe || !pr.ctl) return;
@@ -613,7 +614,7 @@ __device__ __forceinline__ void side_block_a(const float* __restrict__ fin, floa
         if (threadIdx.x == 0) pr.ctl->step[pr.parity ^ 1] = s + 1;
         return;
     }
-    const int p = (pb - 1) * 4 + (int)(threadIdx.x >> 5);
+    const int p = (pb - 1) * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5);
     if (p < pr.n) probe_warp_a(fin, L, a, b, pr, s - pr.ctl->probe_base, p, threadIdx.x & 31);
 }
 
@@ -858,24 +859,38 @@ cudaError_t launch_step_a(const float* fin, float* fout, const Layout& L, const 
     // 208^3 grid 0.309 ms (0.293 ms with the paired collision) against 0.326 ms
     // at 96 registers with four planes per thread, 0.320 ms at 80 registers with
     // two, 0.349-0.367 ms otherwise
-    constexpr int kBlock = kPairBlock;
-    const unsigned gx = (unsigned)((L.nx + 2 * kBlock - 1) / (2 * kBlock));
-    SideBlocks side = side_blocks_a(L, (int)gx, b.copy, pr.n);
+    // (a grid of less than a wave of warps waits for latency, not for warps: 128x128x3 7.5 us a step with half of
+    // every block idle, 8.4 us with blocks of two warps)
+    const bool wave = (long long)((L.nx + 63) / 64) * L.ny * L.nz > 148 * 28;
+    const int warps = wave ? row_block_warps(L.nx) : 4;
+    const unsigned gx = (unsigned)((L.nx + 64 * warps - 1) / (64 * warps));
+    SideBlocks side = side_blocks_a(L, (int)gx, warps, b.copy, pr.n);
     if (!step_a_has_side(b)) side.rows = 0;
     const dim3 grid(gx, (unsigned)(L.ny + side.rows), (unsigned)L.nz);
-    if (!step_a_has_side(b))
-        k_step_a<kBlock, 7, 2, 1, false><<<grid, kBlock, 0, stream>>>(fin, fout, L, a, b, pr, side);
-    else if (b.blend || b.zper)
-        k_step_a<kBlock, 7, 1, 1, true><<<grid, kBlock, 0, stream>>>(fin, fout, L, a, b, pr, side);
-    else
-        k_step_a<kBlock, 7, 0, 1, true><<<grid, kBlock, 0, stream>>>(fin, fout, L, a, b, pr, side);
+    const auto launch = [&](auto w, auto minb) {
+        constexpr int B = 32 * decltype(w)::value, M = decltype(minb)::value;
+        if (!step_a_has_side(b))
+            k_step_a<B, M, 2, 1, false><<<grid, B, 0, stream>>>(fin, fout, L, a, b, pr, side);
+        else if (b.blend || b.zper)
+            k_step_a<B, M, 1, 1, true><<<grid, B, 0, stream>>>(fin, fout, L, a, b, pr, side);
+        else
+            k_step_a<B, M, 0, 1, true><<<grid, B, 0, stream>>>(fin, fout, L, a, b, pr, side);
+    };
+    using std::integral_constant;
+    switch (warps)
+    {
+    case 2: launch(integral_constant<int, 2>{}, integral_constant<int, 14>{}); break;
+    case 3: launch(integral_constant<int, 3>{}, integral_constant<int, 9>{}); break;
+    case 5: launch(integral_constant<int, 5>{}, integral_constant<int, 5>{}); break;
+    default: launch(integral_constant<int, 4>{}, integral_constant<int, 7>{}); break;
+    }
     return cudaGetLastError();
 }
 
 cudaError_t launch_side_a(const float* fin, float* fout, const Layout& L, const StepArgs& a, const SchemeAArgs& b,
                           const ProbeArgs& pr, cudaStream_t stream)
 {
-    const SideBlocks side = side_blocks_a(L, 1, b.copy, pr.n);
+    const SideBlocks side = side_blocks_a(L, 1, kPairBlock / 32, b.copy, pr.n);
     k_side_a<<<dim3((unsigned)side.rows, (unsigned)L.nz), kPairBlock, 0, stream>>>(fin, fout, L, a, b, pr, side);
     return cudaGetLastError();
 }

@@ -19,6 +19,8 @@ pytestmark = pytest.mark.gpu
 TOL = 1e-5
 
 SIZES = [(16, 9, 6), (33, 7, 12), (64, 21, 5), (129, 6, 8), (257, 5, 6)]
+# more warps than a wave holds: blocks of two, three, four and five warps along a row
+WIDE = [(66, 80, 40), (139, 50, 31), (208, 40, 30), (310, 33, 31)]
 
 
 def case(kind, size):
@@ -51,7 +53,7 @@ def case(kind, size):
     return cfg, s, probes, solid.ravel(), cols
 
 
-@pytest.mark.parametrize("size", SIZES, ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("size", SIZES + WIDE, ids=lambda s: "x".join(map(str, s)))
 @pytest.mark.parametrize("kind", ["copy", "copy_flow", "copy_columns", "periodic", "periodic_columns"])
 def test_scheme_a_matches_oracle(kind, size, gpu):
     cfg, src, probes, mask, cols = case(kind, size)
