@@ -293,10 +293,12 @@ __device__ __forceinline__ void source_gradient(const AdjSourceArgs& a)
 // caller's AdjBetweenArgs); blocks [0, nghost) the ghosts, then the residuals,
 // then one for the source.  As launches of their own the last two took a
 // second stream and two event pairs a step.
-__global__ void __launch_bounds__(128, 8) k_adj_between(const __grid_constant__ AdjGhostArgs a,
-                                                     const __grid_constant__ AdjProbeArgs pa,
-                                                     const __grid_constant__ AdjSourceArgs sa, int nghost, int nprobe)
+__global__ void __launch_bounds__(128, 8) k_adj_between(AdjGhostArgs a, const __grid_constant__ AdjProbeArgs pa,
+                                                     AdjSourceArgs sa, int nghost, int nprobe)
 {
+    a.lam_in = chain_wait(a.lam_in);
+    sa.lam_in = after_wait(sa.lam_in);
+    sa.gadj = after_wait(sa.gadj);
     if ((int)blockIdx.x >= nghost)
     {
         const int b = (int)blockIdx.x - nghost;
@@ -434,6 +436,8 @@ __device__ __forceinline__ void adj_prefetch_rows(const AdjStepArgs& a, int j, i
 template <int BLOCK, int MINB>
 __global__ void __launch_bounds__(BLOCK, MINB) k_adj_step(AdjStepArgs a)
 {
+    a.lam_in = chain_wait(a.lam_in);
+    a.gadj = after_wait(a.gadj);
     constexpr int BC = 32;
     const Layout& L = a.L;
     const int lane = threadIdx.x & 31;
@@ -633,9 +637,8 @@ cudaError_t launch_adj_between(const AdjGhostArgs* ghost, const AdjProbeArgs* re
     const int nprobe = resid ? (resid->n + 127) / 128 : 0;
     const int blocks = nghost + nprobe + (source ? 1 : 0);
     if (blocks == 0) return cudaSuccess;
-    k_adj_between<<<blocks, 128, 0, stream>>>(ghost ? *ghost : AdjGhostArgs{}, resid ? *resid : AdjProbeArgs{},
-                                              source ? *source : AdjSourceArgs{}, nghost, nprobe);
-    return cudaGetLastError();
+    return launch_chained(k_adj_between, blocks, 128, 0, stream, ghost ? *ghost : AdjGhostArgs{},
+                          resid ? *resid : AdjProbeArgs{}, source ? *source : AdjSourceArgs{}, nghost, nprobe);
 }
 
 cudaError_t launch_adj_step(const AdjStepArgs& a, cudaStream_t stream)
@@ -646,12 +649,11 @@ cudaError_t launch_adj_step(const AdjStepArgs& a, cudaStream_t stream)
     const dim3 g((unsigned)((a.L.nx + cells - 1) / cells), (unsigned)a.L.ny, (unsigned)a.L.nz);
     switch (warps)
     {
-    case 2: k_adj_step<64, 10><<<g, 64, 0, stream>>>(a); break;
-    case 3: k_adj_step<96, 8><<<g, 96, 0, stream>>>(a); break;
-    case 5: k_adj_step<160, 5><<<g, 160, 0, stream>>>(a); break;
-    default: k_adj_step<128, 6><<<g, 128, 0, stream>>>(a); break;
+    case 2: return launch_chained(k_adj_step<64, 10>, g, 64, 0, stream, a);
+    case 3: return launch_chained(k_adj_step<96, 8>, g, 96, 0, stream, a);
+    case 5: return launch_chained(k_adj_step<160, 5>, g, 160, 0, stream, a);
+    default: return launch_chained(k_adj_step<128, 6>, g, 128, 0, stream, a);
     }
-    return cudaGetLastError();
 }
 
 cudaError_t check_read_adjoint(check::Status* out) { return check::read_and_clear(out); }

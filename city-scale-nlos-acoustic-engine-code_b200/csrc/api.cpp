@@ -1742,7 +1742,10 @@ extern "C" int lbm_step(lbm_handle* h, int nsteps)
             return h->fail(LBM_ERR_NAN, "non-finite probe value by step " + std::to_string(h->step));
         return LBM_OK;
     }
-    const bool use_graph = h->cfg.use_graphs && !h->timing;
+    // FP16 steps are replayed as graphs; FP32 steps are chained launches (launch_chained), which the edges of a
+    // two-step graph do not keep up with: 97x83x41 11.1 us a step chained, 12.4 as graphs, 128^3 64.0 and 65.6,
+    // 01's 320x320x8 29.5 and 30.6; FP16 97x83x41 15.7 as launches, 14.4 as graphs
+    const bool use_graph = h->cfg.use_graphs && !h->timing && h->storage == LBM_STORE_F16;
     long long left = nsteps;
     while (left > 0)
     {

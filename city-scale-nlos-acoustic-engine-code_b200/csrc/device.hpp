@@ -304,6 +304,45 @@ inline int row_block_warps(int nx)
     return best;
 }
 
+#ifdef __CUDACC__
+// Launches that follow one another in a batch are chained by programmatic
+// dependent launch: the next kernel's blocks are placed while the last blocks
+// of this one run, and wait here for all of it before they touch memory.  `f`
+// is the population buffer the kernel reads: passing it through keeps the
+// compiler from moving its read-only loads above the wait.
+template <typename T>
+__device__ __forceinline__ T* chain_wait(T* f)
+{
+    asm volatile("griddepcontrol.wait;" : "+l"(f)::"memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    return f;
+}
+// Another such array of the kernel, after its chain_wait.
+template <typename T>
+__device__ __forceinline__ T* after_wait(T* p)
+{
+    asm volatile("" : "+l"(p)::"memory");
+    return p;
+}
+// Launch that may be placed before the kernel ahead of it in the stream has ended (which then has to call
+// chain_wait before it touches memory).
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t stream, A&&... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+#endif
+
 // ---- launchers (kernels.cu) ----------------------------------------------
 // storage: 0 = float, 1 = __half.  All launches go to `stream`.
 cudaError_t launch_build_links(const uint8_t* mask_ref, uint32_t* links, uint32_t* near, const Layout& L,

@@ -632,6 +632,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_step_a(const float* __restrict_
                                                         Layout L, StepArgs a, SchemeAArgs b,
                                                         const __grid_constant__ ProbeArgs pr, SideBlocks side)
 {
+    fin = chain_wait(fin);
     if constexpr (SIDE)
     {
         const int row0 = (int)gridDim.y - side.rows;
@@ -701,6 +702,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_step_a(const float* __restrict_
 __global__ void __launch_bounds__(kPairBlock) k_side_a(const float* __restrict__ fin, float* __restrict__ fout, Layout L,
                                                        StepArgs a, SchemeAArgs b, ProbeArgs pr, SideBlocks side)
 {
+    fin = chain_wait(fin);
     side_block_a(fin, fout, L, a, b, pr, side, blockIdx.y, blockIdx.x);
 }
 
@@ -869,30 +871,27 @@ cudaError_t launch_step_a(const float* fin, float* fout, const Layout& L, const 
     const dim3 grid(gx, (unsigned)(L.ny + side.rows), (unsigned)L.nz);
     const auto launch = [&](auto w, auto minb) {
         constexpr int B = 32 * decltype(w)::value, M = decltype(minb)::value;
-        if (!step_a_has_side(b))
-            k_step_a<B, M, 2, 1, false><<<grid, B, 0, stream>>>(fin, fout, L, a, b, pr, side);
-        else if (b.blend || b.zper)
-            k_step_a<B, M, 1, 1, true><<<grid, B, 0, stream>>>(fin, fout, L, a, b, pr, side);
-        else
-            k_step_a<B, M, 0, 1, true><<<grid, B, 0, stream>>>(fin, fout, L, a, b, pr, side);
+        const auto kernel = !step_a_has_side(b)    ? k_step_a<B, M, 2, 1, false>
+                            : (b.blend || b.zper) ? k_step_a<B, M, 1, 1, true>
+                                                  : k_step_a<B, M, 0, 1, true>;
+        return launch_chained(kernel, grid, B, 0, stream, fin, fout, L, a, b, pr, side);
     };
     using std::integral_constant;
     switch (warps)
     {
-    case 2: launch(integral_constant<int, 2>{}, integral_constant<int, 14>{}); break;
-    case 3: launch(integral_constant<int, 3>{}, integral_constant<int, 9>{}); break;
-    case 5: launch(integral_constant<int, 5>{}, integral_constant<int, 5>{}); break;
-    default: launch(integral_constant<int, 4>{}, integral_constant<int, 7>{}); break;
+    case 2: return launch(integral_constant<int, 2>{}, integral_constant<int, 14>{});
+    case 3: return launch(integral_constant<int, 3>{}, integral_constant<int, 9>{});
+    case 5: return launch(integral_constant<int, 5>{}, integral_constant<int, 5>{});
+    default: return launch(integral_constant<int, 4>{}, integral_constant<int, 7>{});
     }
-    return cudaGetLastError();
 }
 
 cudaError_t launch_side_a(const float* fin, float* fout, const Layout& L, const StepArgs& a, const SchemeAArgs& b,
                           const ProbeArgs& pr, cudaStream_t stream)
 {
     const SideBlocks side = side_blocks_a(L, 1, kPairBlock / 32, b.copy, pr.n);
-    k_side_a<<<dim3((unsigned)side.rows, (unsigned)L.nz), kPairBlock, 0, stream>>>(fin, fout, L, a, b, pr, side);
-    return cudaGetLastError();
+    return launch_chained(k_side_a, dim3((unsigned)side.rows, (unsigned)L.nz), kPairBlock, 0, stream, fin, fout, L, a, b, pr,
+                          side);
 }
 
 cudaError_t launch_init_a(float* f0, float* f1, float* xgh0, float* xgh1, const uint8_t* mask_ref, const Layout& L,
