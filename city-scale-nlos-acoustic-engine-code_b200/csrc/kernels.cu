@@ -607,6 +607,11 @@ constexpr int kLinkOff = kPopBytes;           // 64 links words
 constexpr int kNearOff = kPopBytes + 256;     // the block's 2 near-solid words
 constexpr int kGhostOff = kNearOff + 16;      // x-face ghosts of a row-end block: 5 per side
 constexpr int kSlotBytes = kGhostOff + 48;
+// A warp's ring has P + 1 slots; of the block before the one being updated it keeps the last words (the
+// directions with ex > 0), in the place of the low x face's ghosts, which only a row's first block has.  With a
+// slot for that block (11.0 instead of 8.3 KB a warp) the L1 cache had 28 KB left, and the bounce-back words of
+// near-solid blocks, up to 18 lines at a time, waited for room in it: a 1024x1024x256 city step 3898 us against
+// 3836.
 // Directions with ex > 0 (ghosts of the low x face) and ex < 0 (high face).
 __device__ __forceinline__ int ghost_dir(int i) { return i < 5 ? (i < 1 ? 1 : i < 3 ? i + 6 : i + 8) : (i < 6 ? 2 : i < 8 ? i + 3 : i + 5); }
 }  // namespace wp
@@ -681,8 +686,8 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
                                                                float inv_scale, const __grid_constant__ FusedArgs fa,
                                                                int side)
 {
-    constexpr int S = P + 2;   // ring slots: blocks t - 1 .. t + P
-    constexpr uint32_t kDirBits = (1u << Q) - 1u;
+    constexpr int S = P + 1;   // ring slots: blocks t .. t + P
+    constexpr uint32_t kDirBits = (1u << Q) - 2u;   // (a SOLID cell's direction 0 pulls its own value anyway)
     extern __shared__ __align__(128) unsigned char wp_smem[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -820,7 +825,6 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
 #pragma unroll 1
     while (cc_r < nrows)
     {
-        const int sp = st == 0 ? S - 1 : st - 1;
         const int sn = st == S - 1 ? 0 : st + 1;
         int si = st + P;
         if (si >= S) si -= S;
@@ -861,9 +865,7 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
 
         // pulled words: line q of the slot, shifted by ex(q) across lanes / blocks
         const unsigned* cur = reinterpret_cast<const unsigned*>(slot) + lane;   // line q: cur[32 q]
-        const unsigned* prv = lane > 0 ? cur - 1
-                                       : (cc_b > 0 ? reinterpret_cast<const unsigned*>(ring + sp * wp::kSlotBytes) + 31
-                                                   : cur);
+        const unsigned* end = reinterpret_cast<const unsigned*>(slot + wp::kGhostOff);   // last words of block t - 1
         const unsigned* nxt =
             lane < 31 ? cur + 1
                       : (cc_b + 1 < L.nb ? reinterpret_cast<const unsigned*>(ring + sn * wp::kSlotBytes) : cur);
@@ -873,14 +875,14 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
         {
             const unsigned v = cur[32 * q];
             if (ex(q) == 0) w[q] = v;
-            else if (ex(q) > 0) w[q] = __byte_perm(prv[32 * q], v, 0x5432);
+            else if (ex(q) > 0) w[q] = __byte_perm(lane > 0 ? cur[32 * q - 1] : end[ghost_slot(q)], v, 0x5432);
             else w[q] = __byte_perm(v, nxt[32 * q], 0x5432);
         }
         if (any_link)
         {
             // halfway bounce-back: the own cell's word of the opposite direction
 #pragma unroll
-            for (int q = 0; q < Q; ++q)
+            for (int q = 1; q < Q; ++q)
             {
                 const unsigned o =
                     ((lka >> q) & 1u) &&
@@ -949,7 +951,10 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
                                  [&](int q) { return last == 0 ? h2f(w[q]).x : h2f(w[q]).y; });
             }
         }
-        __syncwarp();   // every lane is done with slot t - 1 before the next copy lands there
+        if (cc_b + 1 < L.nb && lane < 5)   // the row goes on: its next block's first cells pull this one's last words
+            reinterpret_cast<unsigned*>(ring + sn * wp::kSlotBytes + wp::kGhostOff)[lane] =
+                reinterpret_cast<const unsigned*>(slot)[32 * wp::ghost_dir(lane) + 31];
+        __syncwarp();   // every lane is done with slot t before the next copy lands there
         cc_next();
         st = sn;
     }
@@ -1331,7 +1336,7 @@ dim3 row_grid(const Layout& L) { return dim3((unsigned)((L.nx + 127) / 128), (un
 template <int P, int WARPS, int MINB, int MODE>
 cudaError_t hw_ctas(int* out)
 {
-    constexpr int smem = WARPS * (P + 2) * wp::kSlotBytes;
+    constexpr int smem = WARPS * (P + 1) * wp::kSlotBytes;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -1367,7 +1372,7 @@ cudaError_t launch_hw(const __half* fin, __half* fout, const Layout& L, const St
     const int side = MODE != kPlain ? side_blocks(fa.probe.n, WARPS) : 0;
     const int grid = (int)(need < ctas ? need : ctas) + side;
     // (not chained: with the next launch's blocks waiting on the SMs a 256x128x128 step took 84.9 us, 80.3 without)
-    constexpr size_t smem = WARPS * (P + 2) * wp::kSlotBytes;
+    constexpr size_t smem = WARPS * (P + 1) * wp::kSlotBytes;
     k_step_hw<P, WARPS, MINB, MODE><<<grid, 32 * WARPS, smem, stream>>>(fin, fout, L, a, inv_scale, fa, side);
     return cudaGetLastError();
 }
