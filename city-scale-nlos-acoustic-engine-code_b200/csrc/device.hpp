@@ -71,6 +71,8 @@ struct Control
     // reads the word that another block of the same launch writes
     long long step[2];
     long long last;        // last step of this batch of steps
+    int rows[2];           // FP16 steps: rows claimed so far of the step that reads buffer p; that step clears
+                           // the other word for the next one
     long long table_base;  // step index of source-table row 0
     long long probe_base;  // step index of probe-buffer row 0
     int nonfinite;         // set by the probe kernels when an owned probe reads a non-finite value

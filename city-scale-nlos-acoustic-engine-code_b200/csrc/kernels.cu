@@ -220,7 +220,11 @@ __device__ __forceinline__ void side_block(const S* __restrict__ fin, const Layo
     if (block == 0)
     {
         if (MODE == kFused) prepare_sources(fa.prep, fa.src, s + 2, s + 1 < last, L, a.links, red);
-        if (fa.ctl && threadIdx.x == 0) fa.ctl->step[fa.parity ^ 1] = s + 1;
+        if (fa.ctl && threadIdx.x == 0)
+        {
+            fa.ctl->step[fa.parity ^ 1] = s + 1;
+            fa.ctl->rows[fa.parity ^ 1] = 0;
+        }
         return;
     }
     const int p = (block - 1) * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5);
@@ -680,7 +684,16 @@ __device__ __forceinline__ void ghost_pair(const unsigned (&w)[Q], const float4&
 }
 
 // MODE: as k_step, the first `side` blocks beside the pipelines.
-template <int P, int WARPS, int MINB, int MODE>
+// CLAIM: a warp's first row is given, every further one is claimed from a
+// counter when the copy cursor reaches the last block of the row before it.
+// The SMs do not run at one speed (near-solid rows, distance to memory, the
+// blocks beside the step), and with fixed rows the step waited for the slowest
+// warps: 1024x1024x256 city 3833 -> 3645 us a step (82 -> 86 % of the measured
+// copy bandwidth), 512x512x128 536 -> 522, 256x256x256 310 -> 302.  Which warp
+// updates a row does not change its bits.  With more than P blocks in a row
+// the update cursor is at most one row behind the copy cursor, so one word
+// carries the next row over.
+template <int P, int WARPS, int MINB, int MODE, bool CLAIM>
 __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __restrict__ fin,
                                                                __half* __restrict__ fout, Layout L, StepArgs a,
                                                                float inv_scale, const __grid_constant__ FusedArgs fa,
@@ -706,6 +719,11 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
     const int all_warps = ((int)gridDim.x - (MODE != kPlain ? side : 0)) * WARPS;
     const int r0 = ((int)blockIdx.x - (MODE != kPlain ? side : 0)) * WARPS + warp;   // rows r0, r0 + all_warps, ...; r = (k-1) ny + (j-1)
     if (r0 >= nrows) return;
+    [[maybe_unused]] int claimed = 0;   // lane 0: the claimed row, less all_warps
+    [[maybe_unused]] volatile int* next_row = reinterpret_cast<int*>(ring + wp::kNearOff + 8);   // of the update cursor
+    const auto claim = [&]() {
+        if (lane == 0) claimed = atomicAdd(&fa.ctl->rows[fa.parity], 1);
+    };
 
     // element offsets of this lane's five 16-byte pieces from the destination block
     int poff[5];
@@ -725,13 +743,14 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
                      c_ez[gq] * (L.ny + 2) - c_ey[gq];
 
     // ---- copy cursor: the next block whose lines are copied
-    int ci_r = r0, ci_b = 0;
+    [[maybe_unused]] int ci_r = r0;
+    int ci_b = 0;
     const __half* ci_src = nullptr;     // the block's own position (lines are offset by poff)
     const uint32_t* ci_near = nullptr;  // the block's two near-solid words
     const uint32_t* ci_link = nullptr;  // links words of this lane's two cells
     const float* ci_gh = nullptr;       // this lane's x-face ghost of the row
-    const auto ci_row = [&]() {
-        const int k = 1 + ci_r / L.ny, j = 1 + ci_r - (k - 1) * L.ny;
+    const auto ci_row = [&](int r) {
+        const int k = 1 + r / L.ny, j = 1 + r - (k - 1) * L.ny;
         ci_src = fin + L.elem(0, 1, j, k);
         ci_near = a.near + ((long long)k * (L.ny + 2) + j) * L.words_per_row;
         ci_link = a.links + L.cell(1, j, k) + 2 * lane;
@@ -744,10 +763,23 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
         if (++ci_b == L.nb)
         {
             ci_b = 0;
-            ci_r += all_warps;
-            if (ci_r < nrows) ci_row();
+            if constexpr (CLAIM)
+            {
+                const int r = all_warps + __shfl_sync(kFull, claimed, 0);
+                __syncwarp();   // every lane has read the row before
+                if (lane == 0) *next_row = r;
+                if (r < nrows) ci_row(r);
+                else ci_b = -1;
+            }
+            else
+            {
+                ci_r += all_warps;
+                if (ci_r < nrows) ci_row(ci_r);
+            }
         }
+        if (CLAIM && ci_b == L.nb - 1) claim();
     };
+    const auto ci_more = [&]() { return CLAIM ? ci_b >= 0 : ci_r < nrows; };
     uint32_t n0 = 0u, n1 = 0u;   // near words of the copy cursor's block, loaded one block ahead
     const auto load_near = [&]() {
         n0 = LBM_IN(kChkHwNear, ci_near - a.near, near_extent(L)) ? __ldg(ci_near) : 0u;
@@ -770,16 +802,17 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
     };
 
     // ---- update cursor: the block being updated
-    int cc_r = r0, cc_b = 0, cc_j = 0, cc_k = 0, c0 = 0;
+    [[maybe_unused]] int cc_r = r0;
+    int cc_b = 0, cc_j = 0, cc_k = 0, c0 = 0;
     const unsigned* own = nullptr;   // this lane's word of line 0 of the block (line q: own[32 q])
     unsigned* outp = nullptr;
     float syz = 0.f;
     // FUSED: what the row's results still take: bits 0-7 sources, bits 8-13 the open faces that the row or
     // one of its ends borders, bit 14 the x-face exports of a step that leaves its results as they are
     unsigned todo = 1u << 14;
-    const auto cc_row = [&]() {
-        cc_k = 1 + cc_r / L.ny;
-        cc_j = 1 + cc_r - (cc_k - 1) * L.ny;
+    const auto cc_row = [&](int r) {
+        cc_k = 1 + r / L.ny;
+        cc_j = 1 + r - (cc_k - 1) * L.ny;
         const long long e = L.elem(0, 1, cc_j, cc_k);
         own = reinterpret_cast<const unsigned*>(fin + e) + lane;
         outp = reinterpret_cast<unsigned*>(fout + e) + lane;
@@ -794,6 +827,7 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
             }
         }
     };
+    const auto cc_more = [&]() { return CLAIM ? cc_k > 0 : cc_r < nrows; };
     const auto cc_next = [&]() {
         own += 19 * 32;
         outp += 19 * 32;
@@ -801,17 +835,26 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
         if (++cc_b == L.nb)
         {
             cc_b = 0;
-            cc_r += all_warps;
-            if (cc_r < nrows) cc_row();
+            if constexpr (CLAIM)
+            {
+                const int r = *next_row;
+                if (r < nrows) cc_row(r);
+                else cc_k = 0;
+            }
+            else
+            {
+                cc_r += all_warps;
+                if (cc_r < nrows) cc_row(cc_r);
+            }
         }
     };
 
-    ci_row();
-    cc_row();
+    ci_row(r0);
+    cc_row(r0);
 #pragma unroll 1
     for (int p = 0; p < P; ++p)
     {
-        if (ci_r < nrows)
+        if (ci_more())
         {
             load_near();
             issue(p);
@@ -819,20 +862,20 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
         }
         cp_async_commit();
     }
-    if (ci_r < nrows) load_near();
+    if (ci_more()) load_near();
 
     int st = 0;   // slot of block t
 #pragma unroll 1
-    while (cc_r < nrows)
+    while (cc_more())
     {
         const int sn = st == S - 1 ? 0 : st + 1;
         int si = st + P;
         if (si >= S) si -= S;
-        if (ci_r < nrows)
+        if (ci_more())
         {
             issue(si);
             ci_next();
-            if (ci_r < nrows) load_near();
+            if (ci_more()) load_near();
         }
         cp_async_commit();
         cp_async_wait<P - 1>();   // blocks up to t + 1 have landed
@@ -1332,8 +1375,8 @@ dim3 row_grid(const Layout& L) { return dim3((unsigned)((L.nx + 127) / 128), (un
 
 // Warp-pipelined FP16 step: dynamic shared memory (one ring per warp) and a
 // grid of as many CTAs as the GPU holds at once (every warp then walks rows
-// all_warps apart).  The attribute and the occupancy are set up once per device.
-template <int P, int WARPS, int MINB, int MODE>
+// all_warps apart, or claims them).  The attribute and the occupancy are set up once per device.
+template <int P, int WARPS, int MINB, int MODE, bool CLAIM>
 cudaError_t hw_ctas(int* out)
 {
     constexpr int smem = WARPS * (P + 1) * wp::kSlotBytes;
@@ -1346,7 +1389,7 @@ cudaError_t hw_ctas(int* out)
     std::lock_guard<std::mutex> lock(mu);
     if (!ctas[dev])
     {
-        const auto kernel = k_step_hw<P, WARPS, MINB, MODE>;
+        const auto kernel = k_step_hw<P, WARPS, MINB, MODE, CLAIM>;
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         int per_sm = 0, sms = 0;
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * WARPS, smem);
@@ -1359,21 +1402,21 @@ cudaError_t hw_ctas(int* out)
     return cudaSuccess;
 }
 
-template <int P, int WARPS, int MINB, int MODE>
+template <int P, int WARPS, int MINB, int MODE, bool CLAIM>
 cudaError_t launch_hw(const __half* fin, __half* fout, const Layout& L, const StepArgs& a, float inv_scale,
                       const FusedArgs& fa, cudaStream_t stream)
 {
     // the per-lane source offsets are 32-bit
     if (L.plane_stride + L.row_stride + 19 * 64 > 0x7fffffffLL) return cudaErrorInvalidValue;
     int ctas = 0;
-    const cudaError_t e = hw_ctas<P, WARPS, MINB, MODE>(&ctas);
+    const cudaError_t e = hw_ctas<P, WARPS, MINB, MODE, CLAIM>(&ctas);
     if (e != cudaSuccess) return e;
     const long long need = ((long long)L.ny * L.nz + WARPS - 1) / WARPS;
     const int side = MODE != kPlain ? side_blocks(fa.probe.n, WARPS) : 0;
     const int grid = (int)(need < ctas ? need : ctas) + side;
     // (not chained: with the next launch's blocks waiting on the SMs a 256x128x128 step took 84.9 us, 80.3 without)
     constexpr size_t smem = WARPS * (P + 1) * wp::kSlotBytes;
-    k_step_hw<P, WARPS, MINB, MODE><<<grid, 32 * WARPS, smem, stream>>>(fin, fout, L, a, inv_scale, fa, side);
+    k_step_hw<P, WARPS, MINB, MODE, CLAIM><<<grid, 32 * WARPS, smem, stream>>>(fin, fout, L, a, inv_scale, fa, side);
     return cudaGetLastError();
 }
 
@@ -1448,9 +1491,10 @@ cudaError_t prepare_step(int storage)
 {
     if (storage == 0) return cudaSuccess;
     int ctas = 0;
-    cudaError_t e = hw_ctas<2, 4, 5, kPlain>(&ctas);
-    if (e == cudaSuccess) e = hw_ctas<2, 4, 5, kSide>(&ctas);
-    return e != cudaSuccess ? e : hw_ctas<2, 4, 5, kFused>(&ctas);
+    cudaError_t e = hw_ctas<2, 4, 5, kPlain, false>(&ctas);
+    if (e == cudaSuccess) e = hw_ctas<2, 4, 5, kSide, false>(&ctas);
+    if (e == cudaSuccess) e = hw_ctas<2, 4, 5, kSide, true>(&ctas);
+    return e != cudaSuccess ? e : hw_ctas<2, 4, 5, kFused, false>(&ctas);
 }
 
 namespace {
@@ -1461,7 +1505,19 @@ cudaError_t launch_step_mode(int storage, const void* fin, void* fout, const Lay
     if (storage == 0 && mom) return launch_pair_step<true, MODE>((const float*)fin, (float*)fout, L, a, mom, fa, stream);
     if (storage == 0) return launch_pair_step<false, MODE>((const float*)fin, (float*)fout, L, a, nullptr, fa, stream);
     if (mom) return cudaErrorInvalidValue;
-    return launch_hw<2, 4, 5, MODE>((const __half*)fin, (__half*)fout, L, a, 1.0f / scale, fa, stream);
+    if constexpr (MODE == kSide)
+    {
+        // Claimed rows pay from about ten rows a warp on: 400x350x128 (15 rows) 328 -> 323 us, 900x700x60 (14)
+        // 610 -> 605, 700x300x90 (9) 306 and 306.5, 900x200x50 (3.4) 164 -> 167, and on the fused step's
+        // grids 320x200x100 (7) 113 -> 116, 256x256x128 (11) 148 -> 151: there the order in which the
+        // warps start says which SMs get the last rows, and fixed rows spread those evenly.
+        int ctas = 0;
+        const cudaError_t e = hw_ctas<2, 4, 5, MODE, true>(&ctas);
+        if (e != cudaSuccess) return e;
+        if (fa.ctl && L.nb > 2 && (long long)L.ny * L.nz >= 10LL * 4 * ctas)
+            return launch_hw<2, 4, 5, MODE, true>((const __half*)fin, (__half*)fout, L, a, 1.0f / scale, fa, stream);
+    }
+    return launch_hw<2, 4, 5, MODE, false>((const __half*)fin, (__half*)fout, L, a, 1.0f / scale, fa, stream);
 }
 }  // namespace
 
