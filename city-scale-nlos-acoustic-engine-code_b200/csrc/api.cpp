@@ -1195,7 +1195,9 @@ void scheme_a_args(lbm_handle* h, int parity, bool batched, long long s, StepArg
 // fused / separate, FP32 64^3 10.7 / 16.9 us, 128^3 66.9 / 72.8,
 // 200x160x100 101 / 109, 256x256x128 219 / 224, 333x222x111 247 / 232,
 // 512x512x128 904 / 891; FP16 64^3 11.5 / 21.5, 128^3 51 / 66, 256x256x128
-// 154 / 167, 400x300x128 281 / 282, 512x512x128 562 / 555.
+// 154 / 167, 400x300x128 281 / 282, 512x512x128 562 / 555.  (Taken before FP32
+// launches were chained, 1-2 us less on the small grids, and before large FP16 grids claimed their rows,
+// 2-5 % less on the separate side of grids above the line.)
 bool fused_steps(const lbm_handle* h)
 {
     const long long most = h->storage == LBM_STORE_F16 ? 1LL << 23 : 1LL << 22;

@@ -615,7 +615,7 @@ constexpr int kSlotBytes = kGhostOff + 48;
 // directions with ex > 0), in the place of the low x face's ghosts, which only a row's first block has.  With a
 // slot for that block (11.0 instead of 8.3 KB a warp) the L1 cache had 28 KB left, and the bounce-back words of
 // near-solid blocks, up to 18 lines at a time, waited for room in it: a 1024x1024x256 city step 3898 us against
-// 3836.
+// 3836 (both with fixed rows).
 // Directions with ex > 0 (ghosts of the low x face) and ex < 0 (high face).
 __device__ __forceinline__ int ghost_dir(int i) { return i < 5 ? (i < 1 ? 1 : i < 3 ? i + 6 : i + 8) : (i < 6 ? 2 : i < 8 ? i + 3 : i + 5); }
 }  // namespace wp

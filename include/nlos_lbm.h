@@ -13,10 +13,10 @@
  * the cases the reference reports on stdout and then carries on (STL not
  * loaded, probe inside a solid).  No C++ exceptions cross this boundary.
  * A handle owns one CUDA stream and is not re-entrant: use one handle per
- * host thread.  (The library also runs some small kernels, such as the probe
- * record beside the step, on a second stream of the handle, joined back to
- * the handle's stream before anything reads their results or overwrites
- * their inputs, so work ordered on the handle's stream sees the same order.)
+ * host thread.  (The adjoint also runs the source injection beside the ghost
+ * fill on a second stream of the handle, joined back to the handle's stream
+ * before anything reads its results or overwrites its inputs, so work ordered
+ * on the handle's stream sees the same order.)
  *
  * Lattice: D3Q19 in the reference's family-B velocity order (06:21-31).
  * Populations are stored on the device as deviations g_q = f_q - w_q from the
@@ -136,7 +136,7 @@ typedef struct lbm_config
                                                         100 / (source density amplitude) keeps
                                                         far-field values out of FP16's subnormals */
     int device;                                      /* CUDA device ordinal */
-    int use_graphs;                                  /* replay multi-step runs as CUDA graphs */
+    int use_graphs;                                  /* replay multi-step FP16 runs as CUDA graphs */
     int verbose;                                     /* print the reference's progress lines */
     /* scheme A (01-04 family); ignored by scheme B */
     int scheme;                                      /* LBM_SCHEME_B (default) or LBM_SCHEME_A */
