@@ -350,10 +350,11 @@ cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, unsigned block, size
 cudaError_t launch_build_links(const uint8_t* mask_ref, uint32_t* links, uint32_t* near, const Layout& L,
                                cudaStream_t stream);
 // Source injection of one step; next non-null (first step of a batch of fused steps): also prepares the
-// sources of the step after it.
+// sources of the step after it.  chained (FP32): see launch_chained.
 cudaError_t launch_source(int storage, void* f, const Layout& L, const StepArgs& sa, const SourceArgs& a,
-                          int parity, SourceNext* next, cudaStream_t stream);
-cudaError_t launch_ghost(int storage, void* f, const Layout& L, const GhostArgs& a, cudaStream_t stream);
+                          int parity, SourceNext* next, cudaStream_t stream, bool chained = false);
+cudaError_t launch_ghost(int storage, void* f, const Layout& L, const GhostArgs& a, cudaStream_t stream,
+                         bool chained = false);
 // Moments (rho', jx, jy, jz) of every cell's pulled populations: the
 // forward data of the adjoint's BGK Jacobian, where they enter only through
 // terms of the wave's amplitude (J^2, J / r, 1 / r with r = 1 + rho').  Each

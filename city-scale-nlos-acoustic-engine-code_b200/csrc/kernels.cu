@@ -1099,6 +1099,7 @@ __global__ void __launch_bounds__(512) k_source(S* __restrict__ f, Layout L, Ste
                                                 SourceNext* __restrict__ next)
 {
     __shared__ double red[32];
+    f = chain_wait(f);
     if (blockIdx.x == 1)
     {
         const long long s = a.ctl->step[parity];
@@ -1251,6 +1252,7 @@ __device__ __forceinline__ void ghost_cell(S* __restrict__ f, const Layout& L, c
 template <typename S>
 __global__ void __launch_bounds__(128) k_ghost(S* __restrict__ f, Layout L, GhostArgs a)
 {
+    f = chain_wait(f);
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= a.total) return;
     int fi = 0;
@@ -1535,18 +1537,22 @@ cudaError_t launch_batched_step(int storage, const void* fin, void* fout, const 
 }
 
 cudaError_t launch_source(int storage, void* f, const Layout& L, const StepArgs& sa, const SourceArgs& a,
-                          int parity, SourceNext* next, cudaStream_t stream)
+                          int parity, SourceNext* next, cudaStream_t stream, bool chained)
 {
     const unsigned blocks = next ? 2 : 1;
+    if (storage == 0 && chained)
+        return launch_chained(k_source<float>, dim3(blocks), 512, 0, stream, (float*)f, L, sa, a, parity, next);
     if (storage == 0) k_source<float><<<blocks, 512, 0, stream>>>((float*)f, L, sa, a, parity, next);
     else k_source<__half><<<blocks, 512, 0, stream>>>((__half*)f, L, sa, a, parity, next);
     return cudaGetLastError();
 }
 
-cudaError_t launch_ghost(int storage, void* f, const Layout& L, const GhostArgs& a, cudaStream_t stream)
+cudaError_t launch_ghost(int storage, void* f, const Layout& L, const GhostArgs& a, cudaStream_t stream, bool chained)
 {
     if (a.total <= 0) return cudaSuccess;
     const unsigned blocks = (unsigned)((a.total + 127) / 128);
+    if (storage == 0 && chained)
+        return launch_chained(k_ghost<float>, dim3(blocks), 128, 0, stream, (float*)f, L, a);
     if (storage == 0) k_ghost<float><<<blocks, 128, 0, stream>>>((float*)f, L, a);
     else k_ghost<__half><<<blocks, 128, 0, stream>>>((__half*)f, L, a);
     return cudaGetLastError();

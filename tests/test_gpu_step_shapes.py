@@ -121,3 +121,26 @@ def test_claimed_rows_equal_single_calls(size, gpu):
     assert np.max(np.abs(a.get_rho())) > 0
     a.close()
     b.close()
+
+
+def test_large_f32_batches_equal_single_calls(gpu):
+    """FP32 past the fused step's size: source, ghost fill and step as chained launches."""
+    cfg, srcs, probes, tris = case((199, 151, 145), abi.LBM_STORE_F32, ground=True)
+    a = nlos_lbm.Solver(cfg, srcs, probes, triangles=tris)
+    b = nlos_lbm.Solver(cfg, srcs, probes, triangles=tris)
+    for s in range(12):
+        a.apply_source(s * a.dt)
+        a.exchange_halos()
+        a.step_collision_bgk()
+        a.record_probes()
+    for n in (1, 4, 7):
+        b.step(n)
+    assert np.array_equal(a.get_probes(), b.get_probes())
+    assert np.array_equal(a.get_probe_energy(), b.get_probe_energy())
+    assert np.array_equal(a.get_rho(), b.get_rho())
+    a.step(3)
+    b.step(3)
+    assert np.array_equal(a.get_rho(), b.get_rho())
+    assert np.max(np.abs(a.get_rho())) > 0
+    a.close()
+    b.close()
