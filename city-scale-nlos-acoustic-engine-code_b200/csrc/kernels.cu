@@ -263,22 +263,22 @@ __device__ __forceinline__ void add_sources(float2 (&G)[Q], const SourceNext* __
 // The next step's ghosts of an open y or z face from a pair's results; `ghost`
 // is the pair's place in the halo row.
 template <int AXIS, int SIDE>
-__device__ __forceinline__ void ghost_pair(const float2 (&G)[Q], const float4& m0, const float4& m1, float* ghost)
+__device__ __forceinline__ void ghost_pair(const float2 (&G)[Q], const GhostState& s0, const GhostState& s1, float* ghost)
 {
     constexpr int BC = block_cells(sizeof(float));
     float2 o[Q];
-    nscbc<AXIS, SIDE>(m0, 1.0f, [&](int q) { return G[q].x; }, [&](int q, float v) { o[q].x = v; });
-    nscbc<AXIS, SIDE>(m1, 1.0f, [&](int q) { return G[q].y; }, [&](int q, float v) { o[q].y = v; });
+    nscbc<AXIS, SIDE, float>(s0, 1.0f, [&](int q) { return G[q].x; }, [&](int q, float v) { o[q].x = v; });
+    nscbc<AXIS, SIDE, float>(s1, 1.0f, [&](int q) { return G[q].y; }, [&](int q, float v) { o[q].y = v; });
 #pragma unroll
     for (int q = 0; q < Q; ++q)
         if (inward<AXIS, SIDE>(q)) *reinterpret_cast<float2*>(ghost + q * BC) = o[q];
 }
 // ... and of an open x face, from the cell at the row's end.
-template <int SIDE, typename Get>
-__device__ __forceinline__ void ghost_end(const float4& m, float inv_scale, const FusedArgs& fa, const XFace& xf,
+template <int SIDE, typename S, typename Get>
+__device__ __forceinline__ void ghost_end(const GhostState& s, float inv_scale, const FusedArgs& fa, const XFace& xf,
                                           const Layout& L, int j, int k, Get&& get)
 {
-    nscbc<0, SIDE>(m, inv_scale, get, [&](int q, float v) { fa.xgh_out[xf.gh_index(SIDE, q, j, k, L.ny, L.nz)] = v; });
+    nscbc<0, SIDE, S>(s, inv_scale, get, [&](int q, float v) { fa.xgh_out[xf.gh_index(SIDE, q, j, k, L.ny, L.nz)] = v; });
 }
 
 // Moments of the ghosts' interior cells, for the adjoint: the pair (c0, c0 + 1)
@@ -489,14 +489,15 @@ __global__ void __launch_bounds__(kPairBlock, MODE == kFused ? 6 : 0) k_step(con
             float4 m0 = make_float4(0.f, 0.f, 0.f, 0.f), m1 = m0;
             if (row | (ends & 3u)) m0 = cell_moments([&](int q) { return G[q].x; });
             if (row | (ends & 8u)) m1 = cell_moments([&](int q) { return G[q].y; });
+            const GhostState s0 = ghost_state<float>(m0, 1.0f), s1 = ghost_state<float>(m1, 1.0f);
             // halo rows of the pair; within the buffer, as every pulled row is
-            if (row & 4u) ghost_pair<1, 0>(G, m0, m1, out - rs);
-            if (row & 8u) ghost_pair<1, 1>(G, m0, m1, out + rs);
-            if (row & 16u) ghost_pair<2, 0>(G, m0, m1, out - ps);
-            if (row & 32u) ghost_pair<2, 1>(G, m0, m1, out + ps);
-            if (ends & 1u) ghost_end<0>(m0, 1.0f, fa, a.xf, L, j, k, [&](int q) { return G[q].x; });
+            if (row & 4u) ghost_pair<1, 0>(G, s0, s1, out - rs);
+            if (row & 8u) ghost_pair<1, 1>(G, s0, s1, out + rs);
+            if (row & 16u) ghost_pair<2, 0>(G, s0, s1, out - ps);
+            if (row & 32u) ghost_pair<2, 1>(G, s0, s1, out + ps);
+            if (ends & 1u) ghost_end<0, float>(s0, 1.0f, fa, a.xf, L, j, k, [&](int q) { return G[q].x; });
             if (ends & 10u)
-                ghost_end<1>(xhi0 ? m0 : m1, 1.0f, fa, a.xf, L, j, k, [&](int q) { return xhi0 ? G[q].x : G[q].y; });
+                ghost_end<1, float>(xhi0 ? s0 : s1, 1.0f, fa, a.xf, L, j, k, [&](int q) { return xhi0 ? G[q].x : G[q].y; });
             if (fa.face_mom) keep_face_moments(fa, L, row, ends, c0, j, k, m0, m1);
             return;
         }
@@ -678,8 +679,8 @@ __device__ __forceinline__ void ghost_pair(const unsigned (&w)[Q], const float4&
                                            unsigned* ghost)
 {
     float lo[Q];
-    nscbc<AXIS, SIDE>(m0, inv_scale, [&](int q) { return h2f(w[q]).x; }, [&](int q, float v) { lo[q] = v; });
-    nscbc<AXIS, SIDE>(m1, inv_scale, [&](int q) { return h2f(w[q]).y; },
+    nscbc<AXIS, SIDE, __half>(ghost_state<__half>(m0, inv_scale), inv_scale, [&](int q) { return h2f(w[q]).x; }, [&](int q, float v) { lo[q] = v; });
+    nscbc<AXIS, SIDE, __half>(ghost_state<__half>(m1, inv_scale), inv_scale, [&](int q) { return h2f(w[q]).y; },
                       [&](int q, float v) { ghost[32 * q] = f2h(make_float2(lo[q], v)); });
 }
 
@@ -982,15 +983,17 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
                 float4 m0 = make_float4(0.f, 0.f, 0.f, 0.f), m1 = m0;
                 if (row | (ends & 3u)) m0 = cell_moments([&](int q) { return h2f(w[q]).x; });
                 if (row | (ends & 8u)) m1 = cell_moments([&](int q) { return h2f(w[q]).y; });
-                const int rsw = (int)(L.row_stride >> 1), psw = (int)(L.plane_stride >> 1);
+                // (with 32-bit offsets nvcc 12.9 stored the low faces' rows one row inside the grid in a variant of
+                // this code that kept both cells' GhostState for all faces)
+                const long long rsw = L.row_stride >> 1, psw = L.plane_stride >> 1;
                 if (row & 4u) ghost_pair<1, 0>(w, m0, m1, inv_scale, outp - rsw);
                 if (row & 8u) ghost_pair<1, 1>(w, m0, m1, inv_scale, outp + rsw);
                 if (row & 16u) ghost_pair<2, 0>(w, m0, m1, inv_scale, outp - psw);
                 if (row & 32u) ghost_pair<2, 1>(w, m0, m1, inv_scale, outp + psw);
                 if (ends & 1u)
-                    ghost_end<0>(m0, inv_scale, fa, a.xf, L, j, k, [&](int q) { return h2f(w[q]).x; });
+                    ghost_end<0, __half>(ghost_state<__half>(m0, inv_scale), inv_scale, fa, a.xf, L, j, k, [&](int q) { return h2f(w[q]).x; });
                 if (ends & 10u)
-                    ghost_end<1>(last == 0 ? m0 : m1, inv_scale, fa, a.xf, L, j, k,
+                    ghost_end<1, __half>(ghost_state<__half>(last == 0 ? m0 : m1, inv_scale), inv_scale, fa, a.xf, L, j, k,
                                  [&](int q) { return last == 0 ? h2f(w[q]).x : h2f(w[q]).y; });
             }
         }
@@ -1147,12 +1150,13 @@ __global__ void __launch_bounds__(512) k_source(S* __restrict__ f, Layout L, Ste
 
 // ---------------------------------------------------------------- ghosts
 // G: the populations of cell I in, its ghost's inward directions out
-template <int AXIS, int SIDE>
+template <int AXIS, int SIDE, typename S>
 __device__ __forceinline__ void ghost_values(float (&G)[Q], float inv_scale, float4* face_mom, long long t)
 {
     const float4 m = cell_moments([&](int q) { return G[q]; });
     if (face_mom) face_mom[t] = m;
-    nscbc<AXIS, SIDE>(m, inv_scale, [&](int q) { return G[q]; }, [&](int q, float v) { G[q] = v; });
+    nscbc<AXIS, SIDE, S>(ghost_state<S>(m, inv_scale), inv_scale, [&](int q) { return G[q]; },
+                         [&](int q, float v) { G[q] = v; });
 }
 
 // One face cell (two x-adjacent ones in FP16 y and z faces) of face (AXIS, SIDE).
@@ -1172,7 +1176,7 @@ __device__ __forceinline__ void ghost_cell(S* __restrict__ f, const Layout& L, c
             return;
 #pragma unroll
         for (int q = 0; q < Q; ++q) G[q] = a.xf.xexp[a.xf.exp_index(SIDE, q, j, k, L.ny, L.nz)];
-        ghost_values<AXIS, SIDE>(G, inv_scale, a.face_mom, t);
+        ghost_values<AXIS, SIDE, S>(G, inv_scale, a.face_mom, t);
 #pragma unroll
         for (int q = 0; q < Q; ++q)
             if (inward<AXIS, SIDE>(q)) a.xf.xgh[a.xf.gh_index(SIDE, q, j, k, L.ny, L.nz)] = G[q];
@@ -1214,10 +1218,10 @@ __device__ __forceinline__ void ghost_cell(S* __restrict__ f, const Layout& L, c
             }
         }
         const long long cell = F.first + (long long)vp * F.nu + up;   // the face enumeration of one cell a thread
-        ghost_values<AXIS, SIDE>(G, inv_scale, a.face_mom, cell);
+        ghost_values<AXIS, SIDE, S>(G, inv_scale, a.face_mom, cell);
         if (two)
         {
-            ghost_values<AXIS, SIDE>(G1, inv_scale, a.face_mom, cell + 1);
+            ghost_values<AXIS, SIDE, S>(G1, inv_scale, a.face_mom, cell + 1);
 #pragma unroll
             for (int q = 0; q < Q; ++q)
                 if (inward<AXIS, SIDE>(q)) *reinterpret_cast<__half2*>(B + q * BCH) = __floats2half2_rn(G[q], G1[q]);
@@ -1242,7 +1246,7 @@ __device__ __forceinline__ void ghost_cell(S* __restrict__ f, const Layout& L, c
         S* B = f + L.elem(0, ci, gj, gk);
 #pragma unroll
         for (int q = 0; q < Q; ++q) G[q] = Io<S>::ld(I + q * BC);
-        ghost_values<AXIS, SIDE>(G, inv_scale, a.face_mom, t);
+        ghost_values<AXIS, SIDE, S>(G, inv_scale, a.face_mom, t);
 #pragma unroll
         for (int q = 0; q < Q; ++q)
             if (inward<AXIS, SIDE>(q)) Io<S>::st(B + q * BC, G[q]);
