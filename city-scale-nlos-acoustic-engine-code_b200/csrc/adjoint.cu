@@ -297,6 +297,7 @@ __global__ void __launch_bounds__(128, 8) k_adj_between(AdjGhostArgs a, const __
                                                      AdjSourceArgs sa, int nghost, int nprobe)
 {
     a.lam_in = chain_wait(a.lam_in);
+    a.face_mom = after_wait(a.face_mom);   // (a recompute ends with the ghost fill that writes them)
     sa.lam_in = after_wait(sa.lam_in);
     sa.gadj = after_wait(sa.gadj);
     if ((int)blockIdx.x >= nghost)
