@@ -162,7 +162,8 @@ __host__ __device__ constexpr bool inward(int q)
 }
 
 template <int AXIS, int SIDE>
-__device__ __forceinline__ void adj_ghost_cell(const AdjGhostArgs& a, const GhostFace& F, long long t, int lt)
+__device__ __forceinline__ void adj_ghost_cell(const AdjGhostArgs& a, const float* lam, const float4* face_mom,
+                                               const GhostFace& F, long long t, int lt)
 {
     const int v = lt / F.nu, u = lt - v * F.nu;
     const Layout& L = a.L;
@@ -201,7 +202,7 @@ __device__ __forceinline__ void adj_ghost_cell(const AdjGhostArgs& a, const Ghos
     {
         const int di = gi + ex(q), dj = gj + ey(q), dk = gk + ez(q);
         // only the directions pointing into the interior reach an interior cell
-        lh[q] = inward<AXIS, SIDE>(q) && interior(L, di, dj, dk) ? __ldg(a.lam_in + L.elem(q, di, dj, dk)) : 0.f;
+        lh[q] = inward<AXIS, SIDE>(q) && interior(L, di, dj, dk) ? __ldg(lam + L.elem(q, di, dj, dk)) : 0.f;
     }
     if ((lkn >> qn) & 1u)
     {
@@ -210,7 +211,7 @@ __device__ __forceinline__ void adj_ghost_cell(const AdjGhostArgs& a, const Ghos
             if (inward<AXIS, SIDE>(q)) lh[q] = 0.f;
     }
     // moments of the interior cell the ghost was built from
-    const float4 m = __ldg(a.face_mom + t);
+    const float4 m = __ldg(face_mom + t);
     // J_ghost^T lam = grad_m sum_q lam_q D_q(m), through lam's weighted moments
     LamMoments A{};
 #pragma unroll
@@ -252,7 +253,7 @@ __device__ __forceinline__ void add_residual(const AdjProbeArgs& a, int p)
 // Source gradient of one step: Lam_c = sum_q w_q lamH^s[q](c) over the
 // injection cells; out = (sum_c w_hat_c Lam_c, sum_c dw_hat_c/dpos Lam_c),
 // reduced in FP64, by one block of 128 threads.
-__device__ __forceinline__ void source_gradient(const AdjSourceArgs& a)
+__device__ __forceinline__ void source_gradient(const AdjSourceArgs& a, const float* lam_in, const float* gadj)
 {
     __shared__ double red[4][4];
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
@@ -262,7 +263,7 @@ __device__ __forceinline__ void source_gradient(const AdjSourceArgs& a)
         const AdjSourceCell e = cells[c];
         if (e.i < 0) continue;
         float lg[Q];
-        gather_lam(a.L, a.links, a.lam_in, a.gadj, a.gadj_off, e.i, e.j, e.k, lg);
+        gather_lam(a.L, a.links, lam_in, gadj, a.gadj_off, e.i, e.j, e.k, lg);
         double lam = 0.0;
 #pragma unroll
         for (int q = 0; q < Q; ++q) lam += wd(q) * (double)lg[q];
@@ -290,23 +291,24 @@ __device__ __forceinline__ void source_gradient(const AdjSourceArgs& a)
 // What comes between two adjoint steps, one launch: the ghost adjoints of step
 // s, the probe residuals of step s and the source terms of the step before
 // (s + 1), each where it touches nothing that another of them writes (the
-// caller's AdjBetweenArgs); blocks [0, nghost) the ghosts, then the residuals,
-// then one for the source.  As launches of their own the last two took a
-// second stream and two event pairs a step.
-__global__ void __launch_bounds__(128, 8) k_adj_between(AdjGhostArgs a, const __grid_constant__ AdjProbeArgs pa,
-                                                     AdjSourceArgs sa, int nghost, int nprobe)
+// conditions at launch_adj_between); blocks [0, nghost) the ghosts, then the
+// residuals, then one for the source.  As launches of their own the last two
+// took a second stream and two event pairs a step.  The waited pointers are
+// values of their own: assigning them to a's members copied all of a to the
+// stack of every thread (a.ga.face is indexed at run time), 352 bytes.
+__global__ void __launch_bounds__(128, 8) k_adj_between(const __grid_constant__ AdjGhostArgs a,
+                                                        const __grid_constant__ AdjProbeArgs pa,
+                                                        const __grid_constant__ AdjSourceArgs sa, int nghost, int nprobe)
 {
-    a.lam_in = chain_wait(a.lam_in);
-    a.face_mom = after_wait(a.face_mom);   // (a recompute ends with the ghost fill that writes them)
-    sa.lam_in = after_wait(sa.lam_in);
-    sa.gadj = after_wait(sa.gadj);
+    const float* lam = chain_wait(a.lam_in);
     if ((int)blockIdx.x >= nghost)
     {
         const int b = (int)blockIdx.x - nghost;
         if (b < nprobe) add_residual(pa, b * 128 + (int)threadIdx.x);
-        else source_gradient(sa);
+        else source_gradient(sa, after_wait(sa.lam_in), after_wait(sa.gadj));
         return;
     }
+    const float4* face_mom = after_wait(a.face_mom);   // (a recompute ends with the ghost fill that writes them)
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= a.ga.total) return;
     int fi = 0;
@@ -315,12 +317,12 @@ __global__ void __launch_bounds__(128, 8) k_adj_between(AdjGhostArgs a, const __
     const int lt = (int)(t - F.first);
     switch (F.axis * 2 + F.side)
     {
-    case 0: adj_ghost_cell<0, 0>(a, F, t, lt); break;
-    case 1: adj_ghost_cell<0, 1>(a, F, t, lt); break;
-    case 2: adj_ghost_cell<1, 0>(a, F, t, lt); break;
-    case 3: adj_ghost_cell<1, 1>(a, F, t, lt); break;
-    case 4: adj_ghost_cell<2, 0>(a, F, t, lt); break;
-    default: adj_ghost_cell<2, 1>(a, F, t, lt); break;
+    case 0: adj_ghost_cell<0, 0>(a, lam, face_mom, F, t, lt); break;
+    case 1: adj_ghost_cell<0, 1>(a, lam, face_mom, F, t, lt); break;
+    case 2: adj_ghost_cell<1, 0>(a, lam, face_mom, F, t, lt); break;
+    case 3: adj_ghost_cell<1, 1>(a, lam, face_mom, F, t, lt); break;
+    case 4: adj_ghost_cell<2, 0>(a, lam, face_mom, F, t, lt); break;
+    default: adj_ghost_cell<2, 1>(a, lam, face_mom, F, t, lt); break;
     }
 }
 
