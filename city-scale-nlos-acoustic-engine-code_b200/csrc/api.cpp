@@ -97,7 +97,7 @@ struct lbm_handle
     float* sig = nullptr;              // sig_x | sig_y | sig_z
     XFace xf{nullptr, nullptr};        // x-face exports and (both parities') ghosts
     // x-face ghosts of each population buffer: a batched step reads its own buffer's and writes the next
-    // one's.  A z-slab steps by single calls only and keeps one array, which its messages write into.
+    // one's.  A z-slab's steps are never fused: it keeps one array, which its messages write into.
     float* xgh_par[2] = {nullptr, nullptr};
     int xgh_last = 0;                  // which of them was filled last (lbm_get_f)
     SourceNext* d_next = nullptr;      // [2] sources applied by the batched step that reads buffer 0 / 1
@@ -1198,8 +1198,11 @@ void scheme_a_args(lbm_handle* h, int parity, bool batched, long long s, StepArg
 // 154 / 167, 400x300x128 281 / 282, 512x512x128 562 / 555.  (Taken before FP32
 // launches were chained, 1-2 us less on the small grids, and before large FP16 grids claimed their rows,
 // 2-5 % less on the separate side of grids above the line.)
+// A z-slab's steps are separate launches, batched or not: the halo planes of its cuts and its one array of
+// x-face ghosts belong to the messages of the step at hand.
 bool fused_steps(const lbm_handle* h)
 {
+    if (h->slab) return false;
     const long long most = h->storage == LBM_STORE_F16 ? 1LL << 23 : 1LL << 22;
     return (long long)h->L.nx * h->L.ny * h->L.nz <= most;
 }
@@ -1727,25 +1730,6 @@ extern "C" int lbm_step(lbm_handle* h, int nsteps)
     st = reset_halos_if_dirty(h);
     if (st) return st;
     const int np = h->nprobe();
-    if (h->slab)
-    {
-        // a z-slab takes its halo planes from messages between single calls; steps without them run the
-        // same calls one by one
-        for (int n = 0; n < nsteps; ++n)
-        {
-            st = lbm_apply_source(h, (double)h->step * h->dt);
-            if (!st) st = lbm_exchange_halos(h);
-            if (!st) st = lbm_step_collision_bgk(h);
-            if (!st) st = lbm_record_probes(h);
-            if (st) return st;
-        }
-        CK(cudaMemcpyAsync(&h->ctl_host->nonfinite, &h->ctl->nonfinite, sizeof(int), cudaMemcpyDeviceToHost, h->stream),
-           "probe flag");
-        CK(cudaStreamSynchronize(h->stream), "step sync");
-        if (h->ctl_host->nonfinite)
-            return h->fail(LBM_ERR_NAN, "non-finite probe value by step " + std::to_string(h->step));
-        return LBM_OK;
-    }
     // FP16 steps are replayed as graphs; FP32 steps are chained launches (launch_chained), which the edges of a
     // two-step graph do not keep up with: 97x83x41 11.1 us a step chained, 12.4 as graphs, 128^3 64.0 and 65.6,
     // 01's 320x320x8 29.5 and 30.6; FP16 97x83x41 15.7 as launches, 14.4 as graphs
