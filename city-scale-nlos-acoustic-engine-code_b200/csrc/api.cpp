@@ -1341,7 +1341,7 @@ cudaError_t enqueue_batched_step(lbm_handle* h, int parity, int& kernels)
         StepArgs sa;
         SchemeAArgs b;
         scheme_a_args(h, parity, true, 0, sa, b);
-        if (step_a_has_side(b)) return e;
+        if (step_a_has_side(h->L, b, h->nprobe())) return e;
         e = launch_side_a((const float*)fc, (float*)h->f[parity ^ 1], h->L, sa, b, probe_args(h, true, 0, parity),
                           h->stream);
         kernels++;
@@ -1672,7 +1672,7 @@ extern "C" int lbm_step_collision_bgk(lbm_handle* h)
     CK(cudaSetDevice(h->device), "cudaSetDevice");
     CK(timed_step_launch(h, h->cur, false, h->step), "step kernel");
     h->launches++;
-    if (h->scheme_a() && h->aa.copy && !step_a_has_side(h->aa))
+    if (h->scheme_a() && h->aa.copy && !step_a_has_side(h->L, h->aa, 0))
     {
         StepArgs sa;
         SchemeAArgs b;

@@ -259,25 +259,35 @@ struct SchemeAArgs
 // 97x83x41 step 25.7 and 22.8 us, a gradient step on 128^3 167 and 156 us.
 // The scheme-A and adjoint steps keep their blocks along x: they sit at their
 // register caps and the row index of a split block costs them 1-10 %.
+// `side` blocks beside the step are further rows of blocks of every plane; a
+// split whose rows of blocks pass kMaxGridY with them is not taken (65535 rows
+// of 200 columns run two warps along x).
+constexpr int kMaxGridY = 65535;
 struct PairLaunch
 {
     dim3 grid;
-    int bx;   // 4, 2 or 1
+    int bx;          // 4, 2 or 1
+    int side_rows;   // of grid.y
 };
 constexpr int kPairBlock = 128;
-inline PairLaunch pair_launch(const Layout& L)
+inline PairLaunch pair_launch(const Layout& L, int side)
 {
     const long long seg = (L.nx + 63) / 64;
-    int best = 4;
+    PairLaunch best{};
     long long least = 0;
+    bool best_fits = false;
     for (int bx = 4; bx >= 1; bx /= 2)
     {
         const int by = 4 / bx;
-        const long long warps = ((seg + bx - 1) / bx * bx) * ((L.ny + by - 1) / by * by);
-        if (bx == 4 || warps < least) best = bx, least = warps;
+        const long long gx = (seg + bx - 1) / bx, gy = (L.ny + by - 1) / by, warps = gx * bx * gy * by;
+        const long long rows = (side + gx * L.nz - 1) / (gx * L.nz);
+        const bool fits = gy + rows <= kMaxGridY;
+        if (best_fits && !(fits && warps < least)) continue;
+        best = PairLaunch{dim3((unsigned)gx, (unsigned)(gy + rows), (unsigned)L.nz), bx, (int)rows};
+        least = warps;
+        best_fits = fits;
     }
-    const int by = 4 / best;
-    return PairLaunch{dim3((unsigned)((seg + best - 1) / best), (unsigned)((L.ny + by - 1) / by), (unsigned)L.nz), best};
+    return best;
 }
 #ifdef __CUDACC__
 // Column pair (0-based first column) and row (1-based) of a thread under pair_launch's shape with BX warps along x.
@@ -400,9 +410,9 @@ cudaError_t launch_import_f(int storage, void* f, const double* in, const Layout
 // next step and, where probe.ctl is set (batched steps), the probe record and the step counter; the initial state, and probes / field of a scheme-A state.
 cudaError_t launch_step_a(const float* fin, float* fout, const Layout& L, const StepArgs& a, const SchemeAArgs& b,
                           const ProbeArgs& probe, cudaStream_t stream);
-// Whether launch_step_a's launch holds the halo copies, probes and counter; else launch_side_a follows it
-// (after a single call only where there are copies).
-inline bool step_a_has_side(const SchemeAArgs& b) { return !(b.field_mode == 2 || b.sg_xy || b.fld_xy); }
+// Whether launch_step_a's launch holds the halo copies, `nprobe` probes and the counter; else launch_side_a
+// follows it (after a single call only where there are copies).
+bool step_a_has_side(const Layout& L, const SchemeAArgs& b, int nprobe);
 cudaError_t launch_side_a(const float* fin, float* fout, const Layout& L, const StepArgs& a, const SchemeAArgs& b,
                           const ProbeArgs& probe, cudaStream_t stream);
 cudaError_t launch_init_a(float* f0, float* f1, float* xgh0, float* xgh1, const uint8_t* mask_ref, const Layout& L,

@@ -1430,15 +1430,19 @@ template <bool MOM, int MODE>
 cudaError_t launch_pair_step(const float* fin, float* fout, const Layout& L, const StepArgs& a, PairMoments* mom,
                              const FusedArgs& fa, cudaStream_t stream)
 {
-    const PairLaunch g = pair_launch(L);
-    dim3 grid = g.grid;
-    const int per_row = (int)(grid.x * grid.z);
-    const int side = MODE != kPlain ? (side_blocks(fa.probe.n, kPairBlock / 32) + per_row - 1) / per_row : 0;
-    grid.y += side;
+    const PairLaunch g = pair_launch(L, MODE != kPlain ? side_blocks(fa.probe.n, kPairBlock / 32) : 0);
+    if (g.grid.y > (unsigned)kMaxGridY && MODE != kPlain && fa.probe.n > 0)
+    {
+        // more probes than rows of blocks are left for: they follow the step, whose input it only reads
+        FusedArgs rest = fa;
+        rest.probe.n = 0;
+        const cudaError_t e = launch_pair_step<MOM, MODE>(fin, fout, L, a, mom, rest, stream);
+        return e != cudaSuccess ? e : launch_probe(0, fin, L, a, fa.probe, stream);
+    }
     const auto kernel = g.bx == 4 ? k_step<4, MOM, MODE> : g.bx == 2 ? k_step<2, MOM, MODE> : k_step<1, MOM, MODE>;
     if (MODE != kPlain)
-        return launch_chained(kernel, grid, kPairBlock, 0, stream, fin, fout, L, a, mom, fa, side);
-    kernel<<<grid, kPairBlock, 0, stream>>>(fin, fout, L, a, mom, fa, side);
+        return launch_chained(kernel, g.grid, kPairBlock, 0, stream, fin, fout, L, a, mom, fa, g.side_rows);
+    kernel<<<g.grid, kPairBlock, 0, stream>>>(fin, fout, L, a, mom, fa, g.side_rows);
     return cudaGetLastError();
 }
 

@@ -851,6 +851,31 @@ __global__ void __launch_bounds__(128) k_field_rho_a(const float* __restrict__ f
 
 }  // namespace
 
+namespace {
+// Launch shape of the step: warps per block along a row, blocks per row, and the blocks beside it (none: they are
+// a launch of their own, for 04's instance and where their rows of blocks do not fit gridDim.y any more; the z-halo
+// copies of a layer grow with its plane, so a grid long in y of few layers gets there: 64x40000x1).
+struct StepShape
+{
+    int warps, gx;
+    SideBlocks side;
+};
+StepShape step_a_shape(const Layout& L, const SchemeAArgs& b, int nprobe)
+{
+    // (a grid of less than a wave of warps waits for latency, not for warps: 128x128x3 7.5 us a step with half of
+    // every block idle, 8.4 us with blocks of two warps)
+    const bool wave = (long long)((L.nx + 63) / 64) * L.ny * L.nz > 148 * 28;
+    StepShape s{};
+    s.warps = wave ? row_block_warps(L.nx) : 4;
+    s.gx = (L.nx + 64 * s.warps - 1) / (64 * s.warps);
+    s.side = side_blocks_a(L, s.gx, s.warps, b.copy, nprobe);
+    if (b.field_mode == 2 || b.sg_xy || b.fld_xy || L.ny + (long long)s.side.rows > kMaxGridY) s.side.rows = 0;
+    return s;
+}
+}  // namespace
+
+bool step_a_has_side(const Layout& L, const SchemeAArgs& b, int nprobe) { return step_a_shape(L, b, nprobe).side.rows > 0; }
+
 cudaError_t launch_step_a(const float* fin, float* fout, const Layout& L, const StepArgs& a, const SchemeAArgs& b,
                           const ProbeArgs& pr, cudaStream_t stream)
 {
@@ -861,23 +886,19 @@ cudaError_t launch_step_a(const float* fin, float* fout, const Layout& L, const 
     // 208^3 grid 0.309 ms (0.293 ms with the paired collision) against 0.326 ms
     // at 96 registers with four planes per thread, 0.320 ms at 80 registers with
     // two, 0.349-0.367 ms otherwise
-    // (a grid of less than a wave of warps waits for latency, not for warps: 128x128x3 7.5 us a step with half of
-    // every block idle, 8.4 us with blocks of two warps)
-    const bool wave = (long long)((L.nx + 63) / 64) * L.ny * L.nz > 148 * 28;
-    const int warps = wave ? row_block_warps(L.nx) : 4;
-    const unsigned gx = (unsigned)((L.nx + 64 * warps - 1) / (64 * warps));
-    SideBlocks side = side_blocks_a(L, (int)gx, warps, b.copy, pr.n);
-    if (!step_a_has_side(b)) side.rows = 0;
-    const dim3 grid(gx, (unsigned)(L.ny + side.rows), (unsigned)L.nz);
+    const StepShape shape = step_a_shape(L, b, pr.n);
+    const SideBlocks& side = shape.side;
+    const dim3 grid((unsigned)shape.gx, (unsigned)(L.ny + side.rows), (unsigned)L.nz);
+    const bool columns = b.field_mode == 2 || b.sg_xy || b.fld_xy;
     const auto launch = [&](auto w, auto minb) {
         constexpr int B = 32 * decltype(w)::value, M = decltype(minb)::value;
-        const auto kernel = !step_a_has_side(b)    ? k_step_a<B, M, 2, 1, false>
+        const auto kernel = columns               ? k_step_a<B, M, 2, 1, false>
                             : (b.blend || b.zper) ? k_step_a<B, M, 1, 1, true>
                                                   : k_step_a<B, M, 0, 1, true>;
         return launch_chained(kernel, grid, B, 0, stream, fin, fout, L, a, b, pr, side);
     };
     using std::integral_constant;
-    switch (warps)
+    switch (shape.warps)
     {
     case 2: return launch(integral_constant<int, 2>{}, integral_constant<int, 14>{});
     case 3: return launch(integral_constant<int, 3>{}, integral_constant<int, 9>{});
