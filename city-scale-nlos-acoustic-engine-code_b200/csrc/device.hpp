@@ -351,7 +351,9 @@ cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, unsigned block, size
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    if (e != cudaSuccess) cudaGetLastError();   // returned here, not to the next plain launch
+    return e;
 }
 #endif
 

@@ -48,3 +48,12 @@ def test_every_chained_kernel_waits_for_what_it_reads():
         body = ks[name][1]
         waited = set(re.findall(r"\b(?:chain_wait|after_wait)\(\s*(?:\w+\.)*(\w+)\s*\)", body))
         assert arrays <= waited, (name, arrays - waited)
+
+
+def test_a_refused_chained_launch_leaves_no_error_behind():
+    """cudaLaunchKernelEx returns its error and keeps it as the last one too, where the next plain launch of any
+    handle, which asks for the last error, would find it."""
+    text = open(os.path.join(CSRC, "device.hpp")).read()
+    body = text[text.index("cudaError_t launch_chained("):]
+    body = body[:body.index("\n}\n")]
+    assert "cudaLaunchKernelEx" in body and "cudaGetLastError()" in body
