@@ -2638,6 +2638,7 @@ extern "C" int lbm_adjoint_grad(lbm_handle* h, int nsteps, const double* observe
             fa.src = schedule;
             fa.probe.out = d_pred;
             fa.face_mom = s + 1 < T ? face_mom_of(s + 1) : nullptr;
+            fa.face_total = h->ga.total;
             for (int f = 0; f < h->ga.nfaces; ++f)
                 fa.face_first[h->ga.face[f].axis * 2 + h->ga.face[f].side] = h->ga.face[f].first;
             CK(launch_batched_step(h->storage, h->f[p], h->f[p ^ 1], L, h->step_args(p), h->scale, fa, true, mom_of(s),

@@ -201,6 +201,7 @@ struct FusedArgs
     ProbeArgs probe;           // n = 0: no probe record in this step
     float4* face_mom;          // non-null: moments of the next step's ghosts' interior cells, as GhostArgs::face_mom
     long long face_first[6];   // first ghost of face f in that order
+    long long face_total;      // ghosts of all faces
 };
 
 // Scheme A (the reference's 01-04 family).  The stored state is the

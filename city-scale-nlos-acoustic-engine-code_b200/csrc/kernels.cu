@@ -245,8 +245,8 @@ __device__ __forceinline__ void add_sources(float2 (&G)[Q], const SourceNext* __
         const int row = ((k - b.k0) * b.n + (j - b.j0)) * b.n, d = c0 + 1 - b.i0;
         const bool in0 = d >= 0 && d < b.n, in1 = d + 1 >= 0 && d + 1 < b.n && c0 + 1 < L.nx;
         float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
-        if (in0) a0 = nx->add[s][row + d];
-        if (in1) a1 = nx->add[s][row + d + 1];
+        if (in0 && LBM_IN(kChkSource, row + d, kStencilCells)) a0 = nx->add[s][row + d];
+        if (in1 && LBM_IN(kChkSource, row + d + 1, kStencilCells)) a1 = nx->add[s][row + d + 1];
         if (a0.w != 0.f)
         {
 #pragma unroll
@@ -261,9 +261,10 @@ __device__ __forceinline__ void add_sources(float2 (&G)[Q], const SourceNext* __
 }
 
 // The next step's ghosts of an open y or z face from a pair's results; `ghost`
-// is the pair's place in the halo row.
+// is the pair's place in the halo row of buffer `f`.
 template <int AXIS, int SIDE>
-__device__ __forceinline__ void ghost_pair(const float2 (&G)[Q], const GhostState& s0, const GhostState& s1, float* ghost)
+__device__ __forceinline__ void ghost_pair(const float2 (&G)[Q], const GhostState& s0, const GhostState& s1, float* ghost,
+                                           [[maybe_unused]] const float* f, [[maybe_unused]] long long total)
 {
     constexpr int BC = block_cells(sizeof(float));
     float2 o[Q];
@@ -271,14 +272,18 @@ __device__ __forceinline__ void ghost_pair(const float2 (&G)[Q], const GhostStat
     nscbc<AXIS, SIDE, float>(s1, 1.0f, [&](int q) { return G[q].y; }, [&](int q, float v) { o[q].y = v; });
 #pragma unroll
     for (int q = 0; q < Q; ++q)
-        if (inward<AXIS, SIDE>(q)) *reinterpret_cast<float2*>(ghost + q * BC) = o[q];
+        if (inward<AXIS, SIDE>(q) && LBM_IN(kChkGhost, ghost - f + q * BC, total - 1))
+            *reinterpret_cast<float2*>(ghost + q * BC) = o[q];
 }
 // ... and of an open x face, from the cell at the row's end.
 template <int SIDE, typename S, typename Get>
 __device__ __forceinline__ void ghost_end(const GhostState& s, float inv_scale, const FusedArgs& fa, const XFace& xf,
                                           const Layout& L, int j, int k, Get&& get)
 {
-    nscbc<0, SIDE, S>(s, inv_scale, get, [&](int q, float v) { fa.xgh_out[xf.gh_index(SIDE, q, j, k, L.ny, L.nz)] = v; });
+    nscbc<0, SIDE, S>(s, inv_scale, get, [&](int q, float v) {
+        const long long e = xf.gh_index(SIDE, q, j, k, L.ny, L.nz);
+        if (LBM_IN(kChkGhost, e, xgh_extent(L))) fa.xgh_out[e] = v;
+    });
 }
 
 // Moments of the ghosts' interior cells, for the adjoint: the pair (c0, c0 + 1)
@@ -289,17 +294,19 @@ __device__ __forceinline__ void keep_face_moments(const FusedArgs& fa, const Lay
 {
     const long long xc = (long long)(k - 1) * L.ny + (j - 1), yc = (long long)(k - 1) * L.nx + c0,
                     zc = (long long)(j - 1) * L.nx + c0;
+    const auto put = [&](long long t, const float4& m) {
+        if (LBM_IN(kChkGhost, t, fa.face_total)) fa.face_mom[t] = m;
+    };
 #pragma unroll
     for (int f = 2; f < 6; ++f)
     {
         if (!((row >> f) & 1u)) continue;
-        float4* p = fa.face_mom + fa.face_first[f] + (f < 4 ? yc : zc);
-        p[0] = m0;
-        if (c0 + 1 < L.nx) p[1] = m1;
+        put(fa.face_first[f] + (f < 4 ? yc : zc), m0);
+        if (c0 + 1 < L.nx) put(fa.face_first[f] + (f < 4 ? yc : zc) + 1, m1);
     }
-    if (ends & 1u) fa.face_mom[fa.face_first[0] + xc] = m0;
-    if (ends & 2u) fa.face_mom[fa.face_first[1] + xc] = m0;
-    if (ends & 8u) fa.face_mom[fa.face_first[1] + xc] = m1;
+    if (ends & 1u) put(fa.face_first[0] + xc, m0);
+    if (ends & 2u) put(fa.face_first[1] + xc, m0);
+    if (ends & 8u) put(fa.face_first[1] + xc, m1);
 }
 
 // Open y and z faces that row (j, k) borders.
@@ -491,10 +498,10 @@ __global__ void __launch_bounds__(kPairBlock, MODE == kFused ? 6 : 0) k_step(con
             if (row | (ends & 8u)) m1 = cell_moments([&](int q) { return G[q].y; });
             const GhostState s0 = ghost_state<float>(m0, 1.0f), s1 = ghost_state<float>(m1, 1.0f);
             // halo rows of the pair; within the buffer, as every pulled row is
-            if (row & 4u) ghost_pair<1, 0>(G, s0, s1, out - rs);
-            if (row & 8u) ghost_pair<1, 1>(G, s0, s1, out + rs);
-            if (row & 16u) ghost_pair<2, 0>(G, s0, s1, out - ps);
-            if (row & 32u) ghost_pair<2, 1>(G, s0, s1, out + ps);
+            if (row & 4u) ghost_pair<1, 0>(G, s0, s1, out - rs, fout, L.total);
+            if (row & 8u) ghost_pair<1, 1>(G, s0, s1, out + rs, fout, L.total);
+            if (row & 16u) ghost_pair<2, 0>(G, s0, s1, out - ps, fout, L.total);
+            if (row & 32u) ghost_pair<2, 1>(G, s0, s1, out + ps, fout, L.total);
             if (ends & 1u) ghost_end<0, float>(s0, 1.0f, fa, a.xf, L, j, k, [&](int q) { return G[q].x; });
             if (ends & 10u)
                 ghost_end<1, float>(xhi0 ? s0 : s1, 1.0f, fa, a.xf, L, j, k, [&](int q) { return xhi0 ? G[q].x : G[q].y; });
@@ -659,8 +666,8 @@ __device__ __forceinline__ void add_sources(unsigned (&w)[Q], const SourceNext* 
         const int row = ((k - b.k0) * b.n + (j - b.j0)) * b.n, d = c0 + 1 - b.i0;
         const bool in0 = d >= 0 && d < b.n, in1 = d + 1 >= 0 && d + 1 < b.n && c0 + 1 < L.nx;
         float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
-        if (in0) a0 = nx->add[s][row + d];
-        if (in1) a1 = nx->add[s][row + d + 1];
+        if (in0 && LBM_IN(kChkSource, row + d, kStencilCells)) a0 = nx->add[s][row + d];
+        if (in1 && LBM_IN(kChkSource, row + d + 1, kStencilCells)) a1 = nx->add[s][row + d + 1];
         if (a0.w != 0.f)
         {
 #pragma unroll
@@ -676,12 +683,16 @@ __device__ __forceinline__ void add_sources(unsigned (&w)[Q], const SourceNext* 
 
 template <int AXIS, int SIDE>
 __device__ __forceinline__ void ghost_pair(const unsigned (&w)[Q], const float4& m0, const float4& m1, float inv_scale,
-                                           unsigned* ghost)
+                                           unsigned* ghost, [[maybe_unused]] const __half* f,
+                                           [[maybe_unused]] long long total)
 {
     float lo[Q];
     nscbc<AXIS, SIDE, __half>(ghost_state<__half>(m0, inv_scale), inv_scale, [&](int q) { return h2f(w[q]).x; }, [&](int q, float v) { lo[q] = v; });
     nscbc<AXIS, SIDE, __half>(ghost_state<__half>(m1, inv_scale), inv_scale, [&](int q) { return h2f(w[q]).y; },
-                      [&](int q, float v) { ghost[32 * q] = f2h(make_float2(lo[q], v)); });
+                              [&](int q, float v) {
+                                  if (LBM_IN(kChkGhost, 2 * (ghost - reinterpret_cast<const unsigned*>(f)) + 64 * q, total - 1))
+                                      ghost[32 * q] = f2h(make_float2(lo[q], v));
+                              });
 }
 
 // MODE: as k_step, the first `side` blocks beside the pipelines.
@@ -986,10 +997,10 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
                 // (with 32-bit offsets nvcc 12.9 stored the low faces' rows one row inside the grid in a variant of
                 // this code that kept both cells' GhostState for all faces)
                 const long long rsw = L.row_stride >> 1, psw = L.plane_stride >> 1;
-                if (row & 4u) ghost_pair<1, 0>(w, m0, m1, inv_scale, outp - rsw);
-                if (row & 8u) ghost_pair<1, 1>(w, m0, m1, inv_scale, outp + rsw);
-                if (row & 16u) ghost_pair<2, 0>(w, m0, m1, inv_scale, outp - psw);
-                if (row & 32u) ghost_pair<2, 1>(w, m0, m1, inv_scale, outp + psw);
+                if (row & 4u) ghost_pair<1, 0>(w, m0, m1, inv_scale, outp - rsw, fout, L.total);
+                if (row & 8u) ghost_pair<1, 1>(w, m0, m1, inv_scale, outp + rsw, fout, L.total);
+                if (row & 16u) ghost_pair<2, 0>(w, m0, m1, inv_scale, outp - psw, fout, L.total);
+                if (row & 32u) ghost_pair<2, 1>(w, m0, m1, inv_scale, outp + psw, fout, L.total);
                 if (ends & 1u)
                     ghost_end<0, __half>(ghost_state<__half>(m0, inv_scale), inv_scale, fa, a.xf, L, j, k, [&](int q) { return h2f(w[q]).x; });
                 if (ends & 10u)
