@@ -212,30 +212,36 @@ __device__ __forceinline__ float4 cell_moments(Get&& get)
     return m;
 }
 
-// x / b as IEEE division rounds it, from y = 1 / b rounded: the correction of Markstein (Computation of elementary
-// functions on the IBM RISC System/6000 processor, 1990), exact once the quotient is within one unit of its last
-// place (after the first of the two steps) and no remainder underflows.  FP16 values and their sums are multiples
-// of 2^-24; an FP32 numerator is scaled up for the remainders, which leaves a second rounding to quotients below
-// 2^-126.  Division itself branches on zeros and tiny numerators, as quiet cells have: with it the scatter box
-// 128^3 took 55.9 us a step in FP16 against 50.2, 256x128x128 FP32 127 against 117.
-template <typename S>
+// Quotients as IEEE division rounds them, by Markstein's correction of an approximate one (Computation of
+// elementary functions on the IBM RISC System/6000 processor, 1990): q + y (x - q b), exact where q is within a
+// unit of its last place and the remainder does not underflow.  Division itself branches on zeros and tiny
+// numerators, as quiet cells have: with it the scatter box 128^3 took 55.9 us a step in FP16 against 50.2,
+// 256x128x128 FP32 127 against 117.  Compared with division bit for bit: `quotient` over 2^33 pairs of |x| in
+// 2^-97 .. 2^90 and every x at b = 1 (smaller moments come with a density of 1), `over` for every |x| to 2^98.
+//
+// x / b, y = 1 / b rounded: two steps, the product alone may be two units off.
 __device__ __forceinline__ float quotient(float x, float b, float y)
 {
-    if (sizeof(S) == 4) x = __fmul_rn(x, 0x1p48f);
     float q = __fmul_rn(x, y);
     q = __fmaf_rn(__fmaf_rn(-q, b, x), y, q);
-    q = __fmaf_rn(__fmaf_rn(-q, b, x), y, q);
-    return sizeof(S) == 4 ? __fmul_rn(q, 0x1p-48f) : q;
+    return __fmaf_rn(__fmaf_rn(-q, b, x), y, q);
+}
+// x / c for c = cs or cs^2, z = 1 / c rounded: one step, the remainder scaled up so that it is exact for any x and
+// a quotient below the normal range is rounded once.
+__device__ __forceinline__ float over(float x, float c, float z)
+{
+    const float q = __fmul_rn(x, z);
+    const float r = __fmaf_rn(-__fmul_rn(q, 0x1p28f), c, __fmul_rn(x, 0x1p28f));
+    return __fmaf_rn(r, z * 0x1p-28f, q);
 }
 
 // What the ghosts of cell I take from its moments m, whichever face they lie on: rho', density and velocity, and
-// p / cs with p = cs^2 rho'.  Quotients are rounded once: a product with a rounded reciprocal has a rounding of
-// its own, and an FP16 ghost on the other side of a rounding step is stored one unit away.
+// p / cs with p = cs^2 rho'.  (A product with a rounded reciprocal has a rounding of its own, and an FP16 ghost on
+// the other side of a rounding step is stored one unit away.)
 struct GhostState
 {
     float rho, r, ux, uy, uz, pc;
 };
-template <typename S>
 __device__ __forceinline__ GhostState ghost_state(const float4& m, float inv_scale)
 {
     constexpr float cs = (float)kCs, cs2 = (float)kCs2;
@@ -248,16 +254,16 @@ __device__ __forceinline__ GhostState ghost_state(const float4& m, float inv_sca
     }
     // (taken for every cell: as a branch they cost the FP32 step 16 bytes of spills, 256x128x128 127 us against 117)
     const float iv = __frcp_rn(g.r);
-    g.ux = quotient<S>(m.y, g.r, iv);
-    g.uy = quotient<S>(m.z, g.r, iv);
-    g.uz = quotient<S>(m.w, g.r, iv);
-    g.pc = quotient<S>(__fmul_rn(cs2, g.rho), cs, 1.0f / cs);
+    g.ux = quotient(m.y, g.r, iv);
+    g.uy = quotient(m.z, g.r, iv);
+    g.uz = quotient(m.w, g.r, iv);
+    g.pc = over(__fmul_rn(cs2, g.rho), cs, 1.0f / cs);
     if (!fluid) g.ux = g.uy = g.uz = 0.0f;
     return g;
 }
 
 // Ghost values of the inward directions of face (AXIS, SIDE) from cell I, through put(q, value).
-template <int AXIS, int SIDE, typename S, typename Get, typename Put>
+template <int AXIS, int SIDE, typename Get, typename Put>
 __device__ __forceinline__ void nscbc(const GhostState& g, float inv_scale, Get&& get, Put&& put)
 {
     const auto mul = [](float x, float y) { return __fmul_rn(x, y); };
@@ -271,7 +277,7 @@ __device__ __forceinline__ void nscbc(const GhostState& g, float inv_scale, Get&
     const float un = AXIS == 0 ? ux : (AXIS == 1 ? uy : uz);
     const float w = SIDE == 0 ? sub(un, g.pc) : add(un, g.pc);
     const float unB = mul(0.5f, w);
-    const float rhoB = quotient<S>(mul(SIDE == 0 ? -0.5f * cs : 0.5f * cs, w), cs2, 1.0f / cs2);
+    const float rhoB = over(mul(SIDE == 0 ? -0.5f * cs : 0.5f * cs, w), cs2, 1.0f / cs2);
     const float rB = fma(rhoB, inv_scale, 1.0f);
     const float bx = AXIS == 0 ? unB : ux, by = AXIS == 1 ? unB : uy, bz = AXIS == 2 ? unB : uz;
     // geq(B) - geq(I) = w_q (d0 + c.v + c^T M c), a quadratic form in

@@ -268,19 +268,19 @@ __device__ __forceinline__ void ghost_pair(const float2 (&G)[Q], const GhostStat
 {
     constexpr int BC = block_cells(sizeof(float));
     float2 o[Q];
-    nscbc<AXIS, SIDE, float>(s0, 1.0f, [&](int q) { return G[q].x; }, [&](int q, float v) { o[q].x = v; });
-    nscbc<AXIS, SIDE, float>(s1, 1.0f, [&](int q) { return G[q].y; }, [&](int q, float v) { o[q].y = v; });
+    nscbc<AXIS, SIDE>(s0, 1.0f, [&](int q) { return G[q].x; }, [&](int q, float v) { o[q].x = v; });
+    nscbc<AXIS, SIDE>(s1, 1.0f, [&](int q) { return G[q].y; }, [&](int q, float v) { o[q].y = v; });
 #pragma unroll
     for (int q = 0; q < Q; ++q)
         if (inward<AXIS, SIDE>(q) && LBM_IN(kChkGhost, ghost - f + q * BC, total - 1))
             *reinterpret_cast<float2*>(ghost + q * BC) = o[q];
 }
 // ... and of an open x face, from the cell at the row's end.
-template <int SIDE, typename S, typename Get>
+template <int SIDE, typename Get>
 __device__ __forceinline__ void ghost_end(const GhostState& s, float inv_scale, const FusedArgs& fa, const XFace& xf,
                                           const Layout& L, int j, int k, Get&& get)
 {
-    nscbc<0, SIDE, S>(s, inv_scale, get, [&](int q, float v) {
+    nscbc<0, SIDE>(s, inv_scale, get, [&](int q, float v) {
         const long long e = xf.gh_index(SIDE, q, j, k, L.ny, L.nz);
         if (LBM_IN(kChkGhost, e, xgh_extent(L))) fa.xgh_out[e] = v;
     });
@@ -496,15 +496,15 @@ __global__ void __launch_bounds__(kPairBlock, MODE == kFused ? 6 : 0) k_step(con
             float4 m0 = make_float4(0.f, 0.f, 0.f, 0.f), m1 = m0;
             if (row | (ends & 3u)) m0 = cell_moments([&](int q) { return G[q].x; });
             if (row | (ends & 8u)) m1 = cell_moments([&](int q) { return G[q].y; });
-            const GhostState s0 = ghost_state<float>(m0, 1.0f), s1 = ghost_state<float>(m1, 1.0f);
+            const GhostState s0 = ghost_state(m0, 1.0f), s1 = ghost_state(m1, 1.0f);
             // halo rows of the pair; within the buffer, as every pulled row is
             if (row & 4u) ghost_pair<1, 0>(G, s0, s1, out - rs, fout, L.total);
             if (row & 8u) ghost_pair<1, 1>(G, s0, s1, out + rs, fout, L.total);
             if (row & 16u) ghost_pair<2, 0>(G, s0, s1, out - ps, fout, L.total);
             if (row & 32u) ghost_pair<2, 1>(G, s0, s1, out + ps, fout, L.total);
-            if (ends & 1u) ghost_end<0, float>(s0, 1.0f, fa, a.xf, L, j, k, [&](int q) { return G[q].x; });
+            if (ends & 1u) ghost_end<0>(s0, 1.0f, fa, a.xf, L, j, k, [&](int q) { return G[q].x; });
             if (ends & 10u)
-                ghost_end<1, float>(xhi0 ? s0 : s1, 1.0f, fa, a.xf, L, j, k, [&](int q) { return xhi0 ? G[q].x : G[q].y; });
+                ghost_end<1>(xhi0 ? s0 : s1, 1.0f, fa, a.xf, L, j, k, [&](int q) { return xhi0 ? G[q].x : G[q].y; });
             if (fa.face_mom) keep_face_moments(fa, L, row, ends, c0, j, k, m0, m1);
             return;
         }
@@ -687,8 +687,8 @@ __device__ __forceinline__ void ghost_pair(const unsigned (&w)[Q], const float4&
                                            [[maybe_unused]] long long total)
 {
     float lo[Q];
-    nscbc<AXIS, SIDE, __half>(ghost_state<__half>(m0, inv_scale), inv_scale, [&](int q) { return h2f(w[q]).x; }, [&](int q, float v) { lo[q] = v; });
-    nscbc<AXIS, SIDE, __half>(ghost_state<__half>(m1, inv_scale), inv_scale, [&](int q) { return h2f(w[q]).y; },
+    nscbc<AXIS, SIDE>(ghost_state(m0, inv_scale), inv_scale, [&](int q) { return h2f(w[q]).x; }, [&](int q, float v) { lo[q] = v; });
+    nscbc<AXIS, SIDE>(ghost_state(m1, inv_scale), inv_scale, [&](int q) { return h2f(w[q]).y; },
                               [&](int q, float v) {
                                   if (LBM_IN(kChkGhost, 2 * (ghost - reinterpret_cast<const unsigned*>(f)) + 64 * q, total - 1))
                                       ghost[32 * q] = f2h(make_float2(lo[q], v));
@@ -1002,9 +1002,9 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_step_hw(const __half* __re
                 if (row & 16u) ghost_pair<2, 0>(w, m0, m1, inv_scale, outp - psw, fout, L.total);
                 if (row & 32u) ghost_pair<2, 1>(w, m0, m1, inv_scale, outp + psw, fout, L.total);
                 if (ends & 1u)
-                    ghost_end<0, __half>(ghost_state<__half>(m0, inv_scale), inv_scale, fa, a.xf, L, j, k, [&](int q) { return h2f(w[q]).x; });
+                    ghost_end<0>(ghost_state(m0, inv_scale), inv_scale, fa, a.xf, L, j, k, [&](int q) { return h2f(w[q]).x; });
                 if (ends & 10u)
-                    ghost_end<1, __half>(ghost_state<__half>(last == 0 ? m0 : m1, inv_scale), inv_scale, fa, a.xf, L, j, k,
+                    ghost_end<1>(ghost_state(last == 0 ? m0 : m1, inv_scale), inv_scale, fa, a.xf, L, j, k,
                                  [&](int q) { return last == 0 ? h2f(w[q]).x : h2f(w[q]).y; });
             }
         }
@@ -1161,12 +1161,12 @@ __global__ void __launch_bounds__(512) k_source(S* __restrict__ f, Layout L, Ste
 
 // ---------------------------------------------------------------- ghosts
 // G: the populations of cell I in, its ghost's inward directions out
-template <int AXIS, int SIDE, typename S>
+template <int AXIS, int SIDE>
 __device__ __forceinline__ void ghost_values(float (&G)[Q], float inv_scale, float4* face_mom, long long t)
 {
     const float4 m = cell_moments([&](int q) { return G[q]; });
     if (face_mom) face_mom[t] = m;
-    nscbc<AXIS, SIDE, S>(ghost_state<S>(m, inv_scale), inv_scale, [&](int q) { return G[q]; },
+    nscbc<AXIS, SIDE>(ghost_state(m, inv_scale), inv_scale, [&](int q) { return G[q]; },
                          [&](int q, float v) { G[q] = v; });
 }
 
@@ -1187,7 +1187,7 @@ __device__ __forceinline__ void ghost_cell(S* __restrict__ f, const Layout& L, c
             return;
 #pragma unroll
         for (int q = 0; q < Q; ++q) G[q] = a.xf.xexp[a.xf.exp_index(SIDE, q, j, k, L.ny, L.nz)];
-        ghost_values<AXIS, SIDE, S>(G, inv_scale, a.face_mom, t);
+        ghost_values<AXIS, SIDE>(G, inv_scale, a.face_mom, t);
 #pragma unroll
         for (int q = 0; q < Q; ++q)
             if (inward<AXIS, SIDE>(q)) a.xf.xgh[a.xf.gh_index(SIDE, q, j, k, L.ny, L.nz)] = G[q];
@@ -1229,10 +1229,10 @@ __device__ __forceinline__ void ghost_cell(S* __restrict__ f, const Layout& L, c
             }
         }
         const long long cell = F.first + (long long)vp * F.nu + up;   // the face enumeration of one cell a thread
-        ghost_values<AXIS, SIDE, S>(G, inv_scale, a.face_mom, cell);
+        ghost_values<AXIS, SIDE>(G, inv_scale, a.face_mom, cell);
         if (two)
         {
-            ghost_values<AXIS, SIDE, S>(G1, inv_scale, a.face_mom, cell + 1);
+            ghost_values<AXIS, SIDE>(G1, inv_scale, a.face_mom, cell + 1);
 #pragma unroll
             for (int q = 0; q < Q; ++q)
                 if (inward<AXIS, SIDE>(q)) *reinterpret_cast<__half2*>(B + q * BCH) = __floats2half2_rn(G[q], G1[q]);
@@ -1257,7 +1257,7 @@ __device__ __forceinline__ void ghost_cell(S* __restrict__ f, const Layout& L, c
         S* B = f + L.elem(0, ci, gj, gk);
 #pragma unroll
         for (int q = 0; q < Q; ++q) G[q] = Io<S>::ld(I + q * BC);
-        ghost_values<AXIS, SIDE, S>(G, inv_scale, a.face_mom, t);
+        ghost_values<AXIS, SIDE>(G, inv_scale, a.face_mom, t);
 #pragma unroll
         for (int q = 0; q < Q; ++q)
             if (inward<AXIS, SIDE>(q)) Io<S>::st(B + q * BC, G[q]);
