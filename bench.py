@@ -197,9 +197,9 @@ def measure(name, storage, steps, warmup, device, torch, barrier, reduce_max, ke
     solid = np.count_nonzero(s.get_mask().reshape(nz + 2, ny + 2, nx + 2)[1:-1, 1:-1, 1:-1])
     fluid_fraction = 1.0 - solid / ncell
     s.step(warmup)
-    # the timed steps run as the library runs them (CUDA graphs); the step
-    # kernel's own duration comes from as many further steps with per-launch
-    # events (which replace the graphs by direct launches)
+    # the timed steps run as the library runs them (FP16: CUDA graphs, else chained
+    # launches); the step kernel's own duration comes from as many further steps with
+    # per-launch events, as direct launches
     l0 = s.launch_count
     ms = device_timed_steps(s, steps, torch, barrier)
     launches = s.launch_count - l0

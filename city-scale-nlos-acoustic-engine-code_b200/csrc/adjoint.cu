@@ -535,7 +535,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_adj_step(AdjStepArgs a)
     if (!active) return;
 
     // ---- ghost-adjoint terms of the open faces the pair borders: lamH of a
-    // face cell also holds what the ghost fill took from it (k_adj_ghost),
+    // face cell also holds what the ghost fill took from it (k_adj_between),
     // and J_C^T is applied to the sum.  y and z faces are whole rows (the
     // branch is uniform across the CTA); the x faces touch the row ends.
     {

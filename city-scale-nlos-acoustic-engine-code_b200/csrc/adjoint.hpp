@@ -29,7 +29,7 @@ struct AdjStepArgs
     StepArgs sa;            // links, sponge, omega of the forward step
     const float* lam_in;    // lamF^s, population layout
     float* lam_out;         // lamF^{s-1}
-    const PairMoments* mom_prev;     // moments (rho', J) of F^{s-1}, dense pair order (launch_step_moments)
+    const PairMoments* mom_prev;     // moments (rho', J) of F^{s-1}, dense pair order (launch_step, launch_batched_step)
     const float* gadj;      // ghost-adjoint contributions of step s, per open face
     long long gadj_off[6];  // offset of face f in gadj, -1 = face not open
     int prefetch_rows;      // > 0: each block prefetches into L2 the storage row first read this many rows ahead
@@ -84,7 +84,7 @@ struct AdjProbeArgs
 cudaError_t launch_adj_between(const AdjGhostArgs* ghost, const AdjProbeArgs* resid, const AdjSourceArgs* source,
                                cudaStream_t stream);
 // J_C^T of the gathered lamF^s (plus, at the open faces, the ghost-adjoint
-// terms written by launch_adj_ghost for the same step) over every interior
+// terms written by launch_adj_between for the same step) over every interior
 // cell.
 cudaError_t launch_adj_step(const AdjStepArgs& a, cudaStream_t stream);
 

@@ -1189,15 +1189,18 @@ void scheme_a_args(lbm_handle* h, int parity, bool batched, long long s, StepArg
 
 // Whether a batched scheme-B step is one launch (the next step's sources and
 // ghosts applied to its results) or three (source, ghost fill, step).  One
-// launch saves the small kernels and the gaps between them, 7 us a step and
-// more, but its step kernel is 4-6 % slower (registers, and the x faces' ghosts
-// are one lane's work), so the line lies where the two are equal: measured
-// fused / separate, FP32 64^3 10.7 / 16.9 us, 128^3 66.9 / 72.8,
-// 200x160x100 101 / 109, 256x256x128 219 / 224, 333x222x111 247 / 232,
-// 512x512x128 904 / 891; FP16 64^3 11.5 / 21.5, 128^3 51 / 66, 256x256x128
-// 154 / 167, 400x300x128 281 / 282, 512x512x128 562 / 555.  (Taken before FP32
-// launches were chained, 1-2 us less on the small grids, and before large FP16 grids claimed their rows,
-// 2-5 % less on the separate side of grids above the line.)
+// launch saves the small kernels and the gaps between them; its step kernel is
+// 4-6 % slower (registers, and the x faces' ghosts are one lane's work).  The
+// line lies below where the two meet.  us a step, fused / separate (open box on a ground plane, two sources, 64
+// receivers; chained FP32 launches, FP16 graphs with claimed rows), | the line:
+//   FP32 64^3 9.2 / 18.9, 128^3 62.2 / 71.0, 200x160x100 96 / 107, 160^3 121 / 125, 256x128x128 110 / 121 |
+//        129x200x180 166 / 172, 256x192x100 128 / 139, 320x200x100 168 / 169, 200^3 238 / 243, 333x222x111 235 / 230,
+//        256x256x128 216 / 226, 400x300x100 328 / 309, 512x512x128 826 / 806
+//   FP16 64^3 10.6 / 23.4, 128^3 48 / 66, 320x200x100 107 / 121, 200^3 171 / 189, 256x256x128 141 / 162 |
+//        900x200x50 160 / 162, 128x300x250 195 / 234, 333x222x150 210 / 214, 129x300x300 295 / 330,
+//        400x300x128 260 / 273, 256^3 276 / 299, 512x512x128 497 / 490
+// Past the line one launch would still gain up to 9 % in FP32 to about 8 M
+// cells (333x222x111: -2 %) and up to 17 % in FP16 to some 17 M.
 // A z-slab's steps are separate launches, batched or not: the halo planes of its cuts and its one array of
 // x-face ghosts belong to the messages of the step at hand.
 bool fused_steps(const lbm_handle* h)

@@ -194,9 +194,9 @@ struct FusedArgs
     float* xgh_out;            // x-face ghosts of the next step
     const SourceNext* next;    // sources of the next step
     SourceNext* prep;          // receives those of the step after it
-    Control* ctl;              // step counter and last step; nullptr: direct_step, direct_last
+    Control* ctl;              // step counter and last step; nullptr (never in a fused step): direct_step
     int parity;                // population buffer the step reads
-    long long direct_step, direct_last;
+    long long direct_step;
     SourceArgs src;
     ProbeArgs probe;           // n = 0: no probe record in this step
     float4* face_mom;          // non-null: moments of the next step's ghosts' interior cells, as GhostArgs::face_mom

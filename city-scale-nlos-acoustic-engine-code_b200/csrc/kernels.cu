@@ -53,48 +53,16 @@ struct Io<__half>
     static __device__ __forceinline__ void st(__half* p, float v) { *p = __float2half_rn(v); }
 };
 
-// Two x-adjacent cells as one aligned vector: float2 (8 B) or half2 (4 B).
-// `V` is the raw register form that is shuffled between lanes.
-template <typename S>
-struct PairIo;
-
-template <>
-struct PairIo<float>
+// Two x-adjacent FP32 cells as one aligned vector.
+struct PairIo
 {
     using V = float2;
     static __device__ __forceinline__ V ld(const float* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
     static __device__ __forceinline__ void st(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
-    static __device__ __forceinline__ float2 cvt(V v) { return v; }
-    static __device__ __forceinline__ float hi_of(V v) { return v.y; }
-    static __device__ __forceinline__ float lo_of(V v) { return v.x; }
     // cells (c-1, c) from the previous pair's high element and cur = (c, c+1)
     static __device__ __forceinline__ float2 left(float prev_hi, V cur) { return make_float2(prev_hi, cur.x); }
     // cells (c+1, c+2) from cur = (c, c+1) and the next pair's low element
     static __device__ __forceinline__ float2 right(V cur, float next_lo) { return make_float2(cur.y, next_lo); }
-    static __device__ __forceinline__ float rnd(float v) { return v; }   // value as stored
-};
-
-template <>
-struct PairIo<__half>
-{
-    using V = unsigned;
-    static __device__ __forceinline__ V ld(const __half* p) { return __ldg(reinterpret_cast<const unsigned*>(p)); }
-    static __device__ __forceinline__ void st(__half* p, float2 v)
-    {
-        *reinterpret_cast<__half2*>(p) = __float22half2_rn(v);
-    }
-    static __device__ __forceinline__ float2 cvt(V u)
-    {
-        __half2 h;
-        *reinterpret_cast<unsigned*>(&h) = u;
-        return __half22float2(h);
-    }
-    // the whole 32-bit word is shuffled; the byte permute picks the half
-    static __device__ __forceinline__ unsigned hi_of(V v) { return v; }
-    static __device__ __forceinline__ unsigned lo_of(V v) { return v; }
-    static __device__ __forceinline__ float2 left(unsigned prev, V cur) { return cvt(__byte_perm(prev, cur, 0x5432)); }
-    static __device__ __forceinline__ float2 right(V cur, unsigned next) { return cvt(__byte_perm(cur, next, 0x5432)); }
-    static __device__ __forceinline__ float rnd(float v) { return __half2float(__float2half_rn(v)); }
 };
 
 __device__ __forceinline__ uint32_t near_bits(const StepArgs& a, const Layout& L, int col, int j, int k)
@@ -216,10 +184,9 @@ __device__ __forceinline__ void side_block(const S* __restrict__ fin, const Layo
                                            const FusedArgs& fa, int block, double* red)
 {
     const long long s = fa.ctl ? fa.ctl->step[fa.parity] : fa.direct_step;
-    [[maybe_unused]] const long long last = fa.ctl ? fa.ctl->last : fa.direct_last;
     if (block == 0)
     {
-        if (MODE == kFused) prepare_sources(fa.prep, fa.src, s + 2, s + 1 < last, L, a.links, red);
+        if (MODE == kFused) prepare_sources(fa.prep, fa.src, s + 2, s + 1 < fa.ctl->last, L, a.links, red);
         if (fa.ctl && threadIdx.x == 0)
         {
             fa.ctl->step[fa.parity ^ 1] = s + 1;
@@ -354,7 +321,7 @@ __global__ void __launch_bounds__(kPairBlock, MODE == kFused ? 6 : 0) k_step(con
                                                       const __grid_constant__ FusedArgs fa, int side_rows)
 {
     using S = float;
-    using P = PairIo<S>;
+    using P = PairIo;
     constexpr bool FUSED = MODE == kFused;
     if constexpr (MODE != kPlain) fin = chain_wait(fin);
     if constexpr (MODE != kPlain)
@@ -405,22 +372,22 @@ __global__ void __launch_bounds__(kPairBlock, MODE == kFused ? 6 : 0) k_step(con
         const typename P::V cur = ldp(row + q * BC);
         if (ex(q) == 0)
         {
-            G[q] = P::cvt(cur);
+            G[q] = cur;
         }
         else if (ex(q) > 0)
         {
             // lane 0 sits at the start of a block: its left neighbour pair is
             // the last pair of the previous block
-            auto prev = __shfl_up_sync(kFull, P::hi_of(cur), 1);
-            if (lane == 0) prev = P::hi_of(ldp(row + q * BC - BE + (BC - 2)));
+            auto prev = __shfl_up_sync(kFull, cur.y, 1);
+            if (lane == 0) prev = ldp(row + q * BC - BE + (BC - 2)).y;
             G[q] = P::left(prev, cur);
         }
         else
         {
             // lane 31 sits at the last pair of a block: its right neighbour
             // pair is the first pair of the next block
-            auto next = __shfl_down_sync(kFull, P::lo_of(cur), 1);
-            if (lane == 31) next = P::lo_of(ldp(row + q * BC + BE - (BC - 2)));
+            auto next = __shfl_down_sync(kFull, cur.x, 1);
+            if (lane == 31) next = ldp(row + q * BC + BE - (BC - 2)).x;
             G[q] = P::right(cur, next);
         }
     }
@@ -431,7 +398,7 @@ __global__ void __launch_bounds__(kPairBlock, MODE == kFused ? 6 : 0) k_step(con
         {
             if (((lk0 | lk1) >> q) & 1u)
             {
-                const float2 o = P::cvt(ldp(own + inv(q) * BC));
+                const float2 o = ldp(own + inv(q) * BC);
                 if ((lk0 >> q) & 1u) G[q].x = o.x;
                 if ((lk1 >> q) & 1u) G[q].y = o.y;
             }
@@ -515,9 +482,9 @@ __global__ void __launch_bounds__(kPairBlock, MODE == kFused ? 6 : 0) k_step(con
 #pragma unroll
         for (int q = 0; q < Q; ++q)
         {
-            if (xlo) a.xf.xexp[a.xf.exp_index(0, q, j, k, L.ny, L.nz)] = P::rnd(G[q].x);
-            if (xhi0) a.xf.xexp[a.xf.exp_index(1, q, j, k, L.ny, L.nz)] = P::rnd(G[q].x);
-            if (xhi1) a.xf.xexp[a.xf.exp_index(1, q, j, k, L.ny, L.nz)] = P::rnd(G[q].y);
+            if (xlo) a.xf.xexp[a.xf.exp_index(0, q, j, k, L.ny, L.nz)] = G[q].x;
+            if (xhi0) a.xf.xexp[a.xf.exp_index(1, q, j, k, L.ny, L.nz)] = G[q].x;
+            if (xhi1) a.xf.xexp[a.xf.exp_index(1, q, j, k, L.ny, L.nz)] = G[q].y;
         }
     }
 }
@@ -527,7 +494,12 @@ __global__ void __launch_bounds__(kPairBlock, MODE == kFused ? 6 : 0) k_step(con
 // through the whole update: the moment pass and the update pass each convert
 // a word to float2 right before use, so no 19 x float2 array is ever live and
 // the kernel needs far fewer registers (more warps, more loads in flight).
-__device__ __forceinline__ float2 h2f(unsigned u) { return PairIo<__half>::cvt(u); }
+__device__ __forceinline__ float2 h2f(unsigned u)
+{
+    __half2 h;
+    *reinterpret_cast<unsigned*>(&h) = u;
+    return __half22float2(h);
+}
 __device__ __forceinline__ unsigned f2h(float2 v)
 {
     const __half2 h = __float22half2_rn(v);
